@@ -15,10 +15,11 @@
 //     (mhd.cpp:1483-1506) into the other P buffer together with the ghost images the next step
 //     needs, and folds the next step's dt / c_h candidates (mhd.cpp:1542-1550, 1589-1601) into a
 //     block reduction; the lower z-face flux of its column stays in registers.
-// The slope list is padded per direction to whole warps (no warp mixes two code paths) and handed
-// out per warp from a shared counter; the face list is one unpadded list over all directions,
-// each face read in its rotated frame by direction-generic code.  Masked-off lanes cost the FP64
-// pipe as much as active ones, so padding is paid for in full.  In the FP64 form the warps that
+// The slope list and the face list are unpadded lists over all directions, run by direction-generic
+// code (each face read in its rotated frame); the slopes are handed out per warp from a shared
+// counter.  Masked-off lanes cost the FP64 pipe as much as active ones, so padding would be paid for
+// in full.  In the FP64 form slopes and fluxes are split between the FP64 pipe and pairs of FP32
+// values (face_split.cuh).  In the FP64 form the warps that
 // own no cell start the next plane's phase A as soon as their own faces are formed (a named
 // barrier that only the owner warps wait at), into a second x/y slope buffer and a third z-slope
 // buffer, so their FP64 pipe does not idle while the last faces are formed.
@@ -38,6 +39,7 @@
 #include <cstdio>
 
 #include "common.cuh"
+#include "face_split.cuh"
 #include "fused_args.h"
 #include "mhd_physics.cuh"
 
@@ -200,8 +202,10 @@ __device__ __forceinline__ void recover_cell<double>(const double (&u)[NCONS], d
 #pragma unroll
   for (int n = 0; n < NPRIM; n++) Pout[L.at(NPRIM, n, kk + NGH, jj + NGH, ii + NGH)] = p[n];
   write_ghost_images<double>(Pout, L, bc, ii, jj, kk, p);
-  dtc = cell_dt<double>(p, dx, dy, dz);
-  chc = cell_ch<double>(p);
+  if (!kFast || !cell_speeds_split(p, dx, dy, dz, dtc, chc)) {
+    dtc = cell_dt<double>(p, dx, dy, dz);
+    chc = cell_ch<double>(p);
+  }
   if constexpr (kFast) {  // the same tests on the integer pipe (dtc NaN; chc NaN or inf; rho, p > 0)
     const long long abs_mask = 0x7FFFFFFFFFFFFFFFLL, inf_bits = 0x7FF0000000000000LL;
     if ((__double_as_longlong(dtc) & abs_mask) > inf_bits || (__double_as_longlong(chc) & inf_bits) == inf_bits)
@@ -267,17 +271,16 @@ __device__ __forceinline__ void update_cell(const DivAcc<double>& acc, const dou
                                             int k, double (&u)[NCONS]) {
 #pragma unroll
   for (int m = 0; m < NCONS; m++) u[m] = Uc[m * fs] - dt * acc.s[m];
-  double taui;
-  if constexpr (kFast) {  // integer-pipe min of the (positive) spacings, Newton-reciprocal division
-    const double dhl = imin(imin(a.dxs[i], a.dys[j]), a.dzs[k]);
-    taui = fdiv(0.1 * chd, dhl);
+  if constexpr (kFast) {  // 1 / min of the spacings as the max of their inverses (integer-pipe comparisons)
+    const double inv = imax(imax(a.xinv[i], a.yinv[j]), a.zinv[k]);
+    u[mbps] = u[mbps] * fma(-(dt * (0.1 * chd)), inv, 1.0);
   } else {
     double dhl = a.dxs[i];
     if (a.dys[j] < dhl) dhl = a.dys[j];
     if (a.dzs[k] < dhl) dhl = a.dzs[k];
-    taui = 0.1 * chd / dhl;
+    const double taui = 0.1 * chd / dhl;
+    u[mbps] = u[mbps] * (1.0 - dt * taui);
   }
-  u[mbps] = u[mbps] * (1.0 - dt * taui);
 }
 
 __device__ __forceinline__ void update_cell(const DivAcc<float>& acc, const double* __restrict__ Uc, size_t fs,
@@ -333,6 +336,14 @@ __device__ __forceinline__ void fused_finish_cta(const InstanceDesc* __restrict_
     lc->blocks_done = 0;
     __threadfence();
   }
+}
+
+// The general FP64 face flux as a function of its own, for the faces face_flux_split leaves (and
+// HLLE): kept out of line, so its registers and code stay off the split's path.
+template <bool GEN>
+__device__ __noinline__ void face_flux_general(const double (&pl)[NPRIM], const double (&pr)[NPRIM], double chg,
+                                               int riemann, int rot, double (&f)[NCONS]) {
+  face_flux<double, 0>(pl, pr, glm_const(chg), f, GEN ? riemann : (int)RIEMANN_HLLD, rot);
 }
 
 // MINB: CTAs per SM the register allocation must allow (__launch_bounds__); 2 at 256 threads caps
@@ -463,7 +474,8 @@ k_fused_step(const InstanceDesc* __restrict__ desc, LaunchCtrl* __restrict__ lc)
     int zc = 1, zn = 2, zf = 0;
     if (own) {
       const R *pm2 = plane(kb - 2), *pm1 = plane(kb - 1), *p0 = plane(kb), *pp1 = plane(kb + 1);
-#pragma unroll
+      constexpr int UN = kFast && std::is_same<R, double>::value ? 2 : NPRIM;
+#pragma unroll UN
       for (int n = 0; n < NPRIM; n++) {
         const R a2 = PV(pm2, n, oi, oj), a1 = PV(pm1, n, oi, oj), b0 = PV(p0, n, oi, oj), b1 = PV(pp1, n, oi, oj);
         SLZ(zf, n, oi, oj) = van_leer(b0 - a1, a1 - a2);
@@ -477,11 +489,11 @@ k_fused_step(const InstanceDesc* __restrict__ desc, LaunchCtrl* __restrict__ lc)
     }
     if (kb + 2 <= ke + 1) fill(slot_of(kb + 2));
 
-    // work-list sizes (the slope sub-lists padded to whole warps) and the divisors of their decode
+    // work-list sizes and the divisors of their decode
     const FastDiv dv0(cx), dv1(cx + 1), dv2(cx + 2);
     const int nxs = cy * (cx + 2), nys = (cy + 2) * cx, nzs = cy * cx;
     const int nxf = cy * (cx + 1), nyf = (cy + 1) * cx, nzf = cy * cx;
-    const int pxs = (nxs + 31) & ~31, pys = (nys + 31) & ~31, pzs = (nzs + 31) & ~31;
+    const int nas = nxs + nys + nzs;
 
     // Two barriers per plane.  Phase A writes only slope buffers that the previous plane's phase C
     // does not read, and phase C reads no ring plane, so neither the start nor the end of a plane
@@ -493,7 +505,7 @@ k_fused_step(const InstanceDesc* __restrict__ desc, LaunchCtrl* __restrict__ lc)
     // that plane k-1's faces read) while the owners' and other warps' last faces are formed.  On the
     // first plane of a chunk everyone waits, and again after the owners have taken the flux through
     // face kb-1/2, whose buffer the next plane's z slopes reuse.
-    const int nwa = (pxs + pys + pzs) >> 5;
+    const int nwa = (nas + 31) >> 5;
     for (int k = kb; k < ke; k++) {
       if constexpr (S::OV) {
         slxk = slx + (k & 1) * (size_t)S::NSLX;
@@ -513,34 +525,40 @@ k_fused_step(const InstanceDesc* __restrict__ desc, LaunchCtrl* __restrict__ lc)
         w = __shfl_sync(0xffffffffu, w, 0);
         if (w >= nwa) break;
         const int q = (w << 5) | (tid & 31);
-        if (q < pxs) {
+        if (q < nas) {
+          // one unpadded list over the x, y and z slopes; every direction runs the same loop, whose
+          // code stays small enough for the instruction caches (unrolled over the 12 variables and
+          // three directions the FP64 slopes alone were several times as long)
+          const R *cm, *c0, *cp;  // variable 0 of the cells below, at and above
+          R* so;
+          int ostr;
           if (q < nxs) {
             const int j = dv2.div(q), i = q - j * (cx + 2) - 1;
-#pragma unroll
-            for (int n = 0; n < NPRIM; n++) {
-              const R m1 = PV(pk, n, i - 1, j), c0 = PV(pk, n, i, j), p1 = PV(pk, n, i + 1, j);
-              SLX(n, i, j) = van_leer(p1 - c0, c0 - m1);
-            }
+            c0 = &PV0(pk, i, j);
+            cm = c0 - 1;
+            cp = c0 + 1;
+            so = &SLX(0, i, j);
+            ostr = TY * (TX + 2);
+          } else if (q < nxs + nys) {
+            const int r = q - nxs, jr = dv0.div(r), j = jr - 1, i = r - jr * cx;
+            c0 = &PV0(pk, i, j);
+            cm = c0 - NPRIM * PX;
+            cp = c0 + NPRIM * PX;
+            so = &SLY(0, i, j);
+            ostr = (TY + 2) * TX;
+          } else {
+            const int r = q - nxs - nys, j = dv0.div(r), i = r - j * cx;
+            cm = &PV0(pk, i, j);
+            c0 = &PV0(pk1, i, j);
+            cp = &PV0(pk2, i, j);
+            so = &SLZ(zn, 0, i, j);
+            ostr = TY * TX;
           }
-        } else if (q < pxs + pys) {
-          const int r = q - pxs;
-          if (r < nys) {
-            const int jr = dv0.div(r), j = jr - 1, i = r - jr * cx;
-#pragma unroll
-            for (int n = 0; n < NPRIM; n++) {
-              const R m1 = PV(pk, n, i, j - 1), c0 = PV(pk, n, i, j), p1 = PV(pk, n, i, j + 1);
-              SLY(n, i, j) = van_leer(p1 - c0, c0 - m1);
-            }
-          }
-        } else {
-          const int r = q - pxs - pys;
-          if (r < nzs) {
-            const int j = dv0.div(r), i = r - j * cx;
-#pragma unroll
-            for (int n = 0; n < NPRIM; n++) {
-              const R c0 = PV(pk, n, i, j), c1 = PV(pk1, n, i, j), c2 = PV(pk2, n, i, j);
-              SLZ(zn, n, i, j) = van_leer(c2 - c1, c1 - c0);
-            }
+          constexpr int UN = kFast && std::is_same<R, double>::value ? 3 : NPRIM;
+#pragma unroll UN
+          for (int n = 0; n < NPRIM; n++) {
+            const R c = c0[n * PX];
+            so[n * ostr] = van_leer(cp[n * PX] - c, c - cm[n * PX]);
           }
         }
       }
@@ -610,7 +628,19 @@ k_fused_step(const InstanceDesc* __restrict__ desc, LaunchCtrl* __restrict__ lc)
             pl[n] = left_state(pa[v * PX], sa[v * sstr]);
             pr[n] = right_state(pb[v * PX], sb[v * sstr]);
           }
-          face_flux<R, 0>(pl, pr, glm, f, riemann, rot);
+          if constexpr (kFast && std::is_same<R, double>::value) {
+            if (riemann == RIEMANN_HLLE ||
+                !face_flux_split(pl, pr, glm.chg, glm.hoc, glm.chg2, f, riemann == RIEMANN_HLLC)) {
+              double a[NPRIM], b[NPRIM], c[NCONS];  // copies: only this path puts them in local memory
+#pragma unroll
+              for (int n = 0; n < NPRIM; n++) { a[n] = pl[n]; b[n] = pr[n]; }
+              face_flux_general<GEN>(a, b, chg, riemann, rot, c);
+#pragma unroll
+              for (int m = 0; m < NCONS; m++) f[m] = c[m];
+            }
+          } else {
+            face_flux<R, 0>(pl, pr, glm, f, riemann, rot);
+          }
           auto slot_of_flux = [&](int m) {
             if (m == mrv1 || m == mbm1) return m + rot;
             if (m == mrv2 || m == mbm2) return m - 1 + c1;

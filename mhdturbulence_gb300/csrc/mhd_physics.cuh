@@ -22,6 +22,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "face_split.cuh"
 
 namespace mhdgb {
 namespace MHDGB_VNS {
@@ -213,12 +214,18 @@ __device__ __forceinline__ double twice_div_est(double p, double s) {
 // van_leer(P[c+1]-P[c], P[c]-P[c-1]); the reference evaluates the same expression for the left
 // state of face c+1/2 and the right state of face c-1/2 (mhd.cpp:1134-1154), so one evaluation
 // per cell and direction gives both.
+// van_leer_general: the FP64 fast build's expression for the arguments van_leer_split leaves, out of line.
+__device__ __noinline__ double van_leer_general(double dsvp, double dsvm) {
+  const double p = dsvp * dsvm;
+  return pos_nonzero(p) ? twice_div_est(p, dsvp + dsvm) : 0.0;
+}
 template <class R>
 __device__ __forceinline__ R van_leer(R dsvp, R dsvm) {
   if constexpr (kFast) {  // one product for the test and the numerator: p + p == (2 dsvp) dsvm exactly
-    const R p = dsvp * dsvm;
+    [[maybe_unused]] const R p = dsvp * dsvm;
     if constexpr (std::is_same<R, double>::value) {
-      return pos_nonzero(p) ? twice_div_est(p, dsvp + dsvm) : R(0);
+      double s;
+      return van_leer_split(dsvp, dsvm, s) ? s : van_leer_general(dsvp, dsvm);
     } else {  // FP32: (p + p) times the MUFU reciprocal, the form the paired evaluation repeats
       return (p > R(0)) ? (p + p) * rcp_approx_f32(dsvp + dsvm) : R(0);
     }
