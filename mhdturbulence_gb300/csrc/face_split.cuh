@@ -19,12 +19,17 @@
 // with _o the other side, J the star states' jump from this side to the other and h = +-1 the sign of
 // B_n as seen from this side.  These are the reference's HLLD states (mhd.cpp:97-417) rearranged.
 //
-// Measured on the FP64 fused step (KH 150^3): 2.68 -> 1.27 ns per cell and step, FP64-pipe instructions
-// 1350 -> 442 per cell, with the limited slopes and the dt / c_h candidates below in pairs too.  The
-// error against the step in 64 bits is no larger: 2.6e-17 -> 2.5e-17 of the state after one step of
-// that grid, 3.4e-17 -> 3.2e-17 on 256^3 turbulence.  On random faces the flux is nearer to the exact
-// one than the reference's expressions evaluated in FP64 while jumps stay below a tenth of the state,
-// and within twice their error at jumps of half the state.
+// What bounds it: a warp's FP64 instruction keeps its sub-partition's FP64 path busy for 65 cycles
+// (19 per instruction and SM with all four in use), so a face costs about 67 x 76 cycles of that
+// path and, beside it, 2200 other instructions.  Hence nothing here that the pairs can hold is FP64, the
+// corrections enter as the innermost addend of the flux's last FMAs, and there are no branches before
+// the end, so that one face's conversions, pair chains and FP64 instructions overlap.
+//
+// Measured on the FP64 fused step (KH 150^3 / 256^3): 2.68 / 2.57 -> 1.09 / 1.02 ns per cell and step,
+// FP64-pipe instructions 1350 -> 394 per cell, with the limited slopes and the dt / c_h candidates below
+// in pairs too (1.27 / 1.21 with renormalised pairs, branches and two subtractions per slope).
+// Against the step in 64 bits the error over the Kelvin-Helmholtz, turbulence and smooth states at CFL
+// 0.05 and 0.3 is 0.46 to 1.04 times that of the FP64 expressions it replaced (geometric mean 0.86).
 #pragma once
 
 #include "fp32pair.cuh"
@@ -41,10 +46,13 @@ constexpr unsigned kSplitMax = (1023u + 20u) << 20, kSplitMin = (1023u - 20u) <<
 MHDGB_HD unsigned d_mag(double d) { return d_hi(d) & 0x7FFFFFFFu; }
 
 // Flux through a face from its reconstructed states (rotated: normal component first), HLLD or, with
-// hllc, HLLC; returns false without touching F where the split does not apply.
-MHDGB_HD bool face_flux_split(const double (&Pl)[NPRIM], const double (&Pr)[NPRIM], double chg, double hoc, double chg2,
-                              double (&F)[NCONS], bool hllc) {
-  // range of the inputs
+// hllc, HLLC; returns false where the split does not apply (F is then meaningless).  hchg = c_h / 2, chg2 =
+// c_h^2 (the GLM pair, mhd.cpp:1234-1237).  The energy and the scalar are wanted on the upwind side only:
+// up(n, left) gives them (their slots of Pl and Pr are not read).
+template <class UP>
+MHDGB_HD bool face_flux_split(const double (&Pl)[NPRIM], const double (&Pr)[NPRIM], const UP& up, double hchg,
+                              double chg2, double (&F)[NCONS], bool hllc) {
+  bool ok;  // (checked at the end: a branch here would keep the loads and conversions below from overlapping)
   {
     unsigned mx = 0, mb = 0xFFFFFFFFu;
     const int q[] = {nve1, nve2, nve3, nbm1, nbm2, nbm3, nden, ncsp};
@@ -57,7 +65,7 @@ MHDGB_HD bool face_flux_split(const double (&Pl)[NPRIM], const double (&Pr)[NPRI
     const int mn = (int)kSplitMin;
     const bool pos = (int)d_hi(Pl[nden]) >= mn && (int)d_hi(Pr[nden]) >= mn && (int)d_hi(Pl[ncsp]) >= mn &&
                      (int)d_hi(Pr[ncsp]) >= mn;
-    if (mx >= kSplitMax || mb < kSplitTinyB || !pos) return false;
+    ok = mx < kSplitMax && mb >= kSplitTinyB && pos;
   }
   const Pair rl = p_narrow_nz(Pl[nden]), rr = p_narrow_nz(Pr[nden]);
   const Pair bxl = p_narrow(Pl[nbm1]), bxr = p_narrow(Pr[nbm1]);
@@ -66,25 +74,26 @@ MHDGB_HD bool face_flux_split(const double (&Pl)[NPRIM], const double (&Pr)[NPRI
   const Pair vxl = p_narrow(Pl[nve1]), vxr = p_narrow(Pr[nve1]);
   const Pair dvx = p_narrow(Pr[nve1] - Pl[nve1]);
   const Pair dby = p_narrow(Pr[nbm2] - Pl[nbm2]), dbz = p_narrow(Pr[nbm3] - Pl[nbm3]);
-  const double jb = Pr[nbm1] - Pl[nbm1], hb = 0.5 * (Pl[nbm1] + Pr[nbm1]);
-  const Pair dbx = p_narrow(jb), bx = p_narrow(hb);
+  const double jb = Pr[nbm1] - Pl[nbm1], hb = d_half(Pl[nbm1] + Pr[nbm1]);
+  const Pair dbx = p_narrow(jb), bxs = p_add(bxl, bxr), bx = p_scale(bxs, 0.5f);
 
   // fast speeds: c_f^2 = (a + b + sqrt((a-b)^2 + t (t + 2(a+b)))) / 2 with a = c_s^2, b = B_n^2/rho,
   // t = B_t^2/rho (the discriminant as a sum of squares, without cancellation)
   const Pair bt2l = p_add(p_sqr(byl), p_sqr(bzl)), bt2r = p_add(p_sqr(byr), p_sqr(bzr));
-  auto fast = [](Pair rho, Pair cs, Pair bn, Pair bt2) {
+  auto fast2 = [](Pair rho, Pair cs, Pair bn, Pair bt2) {  // c_f^2
     const Pair ri = p_rcp(rho), a = p_sqr(cs), b = p_mul(p_sqr(bn), ri), t = p_mul(bt2, ri);
-    const Pair s = p_add(a, b), d = p_sub(a, b);
+    const Pair s = p_add(a, b), d = p_norm(p_sub(a, b));
     const Pair disc = p_fma(t, p_add(t, p_scale(s, 2.0f)), p_sqr(d));
-    return p_sqrt(p_scale(p_add(p_add(s, t), p_sqrt(disc)), 0.5f));
+    return p_scale(p_add(p_add(s, t), p_sqrt(disc)), 0.5f);
   };
-  const Pair cm = p_max(fast(rl, p_narrow_nz(Pl[ncsp]), bxl, bt2l), fast(rr, p_narrow_nz(Pr[ncsp]), bxr, bt2r));
-  const Pair w = dvx.h < 0.0f ? p_sub(cm, dvx) : cm;
+  const Pair cm = p_sqrt(p_max(fast2(rl, p_narrow_nz(Pl[ncsp]), bxl, bt2l), fast2(rr, p_narrow_nz(Pr[ncsp]), bxr, bt2r)));
+  const Pair w = p_norm(dvx.h < 0.0f ? p_sub(cm, dvx) : cm);
 
-  // contact speed, and relative to the sides
+  // contact speed, and relative to the sides (the results that the largest corrections are proportional
+  // to are normalised: that takes a quarter off the error of the mass and energy fluxes)
   Pair dp = p_narrow(Pr[npre] - Pl[npre]);
   {
-    Pair db2 = p_mul(dbx, p_add(bxl, bxr));
+    Pair db2 = p_mul(dbx, bxs);
     db2 = p_fma(dby, p_add(byl, byr), db2);
     db2 = p_fma(dbz, p_add(bzl, bzr), db2);
     dp = p_add(dp, p_scale(db2, 0.5f));
@@ -93,45 +102,43 @@ MHDGB_HD bool face_flux_split(const double (&Pl)[NPRIM], const double (&Pr)[NPRI
   // mirror-image states (a reflecting wall) give exactly zero here, and the left side is taken, as
   // in the reference (its fluxes on the two sides of S_M = 0 differ when B_n != 0)
   const Pair sm = p_mul(p_sub(p_fma(rr, vxr, p_mul(rl, vxl)), dpw), ir);
-  const bool left = !(sm.h < 0.0f);
-  const Pair dl = p_mul(p_sub(p_mul(rr, dvx), dpw), ir);
-  const Pair dr = p_neg(p_mul(p_fma(rl, dvx, dpw), ir));
+  const bool left = !(f_add(sm.h, sm.l) < 0.0f);
+  const Pair dl = p_norm(p_mul(p_norm(p_sub(p_mul(rr, dvx), dpw)), ir));
+  const Pair dr = p_sub(dl, dvx);
 
   // upwind side; signs as seen from it (x_: times +1 on the left, -1 on the right)
   const double rho = left ? Pl[nden] : Pr[nden], vx = left ? Pl[nve1] : Pr[nve1], vy = left ? Pl[nve2] : Pr[nve2],
                vz = left ? Pl[nve3] : Pr[nve3], bxu = left ? Pl[nbm1] : Pr[nbm1], by = left ? Pl[nbm2] : Pr[nbm2],
                bz = left ? Pl[nbm3] : Pr[nbm3];
   const double bsq = fma(bz, bz, fma(by, by, bxu * bxu)), vsq = fma(vz, vz, fma(vy, vy, vx * vx));
-  const double en = fma(0.5, bsq, rho * fma(0.5, vsq, left ? Pl[nene] : Pr[nene]));
-  const double pt = fma(0.5, bsq, left ? Pl[npre] : Pr[npre]);
-  const double ep = en + pt, m = rho * vx;
+  const double pu = left ? Pl[npre] : Pr[npre], pt = fma(0.5, bsq, pu), m = rho * vx;
+  const double ep = fma(rho, fma(0.5, vsq, up(nene, left)), pu + bsq);  // E + p_T
 
   const Pair ru = p_sel(left, rl, rr), ro = p_sel(left, rr, rl);
   const Pair byu = p_sel(left, byl, byr), bzu = p_sel(left, bzl, bzr);
   const Pair vyu = p_narrow(vy), vzu = p_narrow(vz);
   const Pair tau = p_neg_if(p_sel(left, dl, dr), !left);
-  const Pair wm = p_add(w, tau);
+  const Pair wm = p_norm(p_add(w, tau));
   const Pair sms = p_neg_if(sm, !left), vs = p_neg_if(p_sel(left, vxl, vxr), !left), bs = p_neg_if(bx, !left);
   const Pair tauo = p_neg_if(p_sel(left, dr, dl), left);
-  const Pair wmo = p_add(w, tauo);
-  if (!(wm.h > 0x1p-10f * w.h) || !(wmo.h > 0x1p-10f * w.h)) return false;
+  const Pair wmo = p_norm(p_add(w, tauo));
+  ok = ok && wm.h > 0x1p-10f * w.h && wmo.h > 0x1p-10f * w.h;
 
   const Pair iwm = p_rcp(wm);
   // T = N + rho w tau with N = rho w^2 - B_n^2 in FP64: near B_t = 0 the fast speed is close to the
   // Alfven speed and N cancels, and a star state needs T and N as consistent as FP64 makes them
   // (an error of w itself only moves the outer wave)
-  const double wd = p_join(w), bb = hb * hb;
-  const double rwd = rho * wd;
-  const Pair rw = p_narrow_nz(rwd);
-  const Pair ti = p_mul(tau, iwm);
-  Pair r1 = p_mul(ru, ti);        // rho - rho*
+  const double wd = p_join(w), w2 = wd * wd, bb = hb * hb;
+  const Pair rw = p_mul(ru, w);
+  const Pair ti = p_norm(p_mul(tau, iwm));
+  Pair r1 = p_norm(p_mul(ru, ti));        // rho - rho*
   Pair f = p_make(0.0f), g, g1;   // v_t* = v_t + f B_t, B_t* = g1 B_t = B_t + g B_t
   bool nondeg = true;
   if (hllc) {
     g = p_neg(ti);
     g1 = p_add(g, p_make(1.0f));
   } else {
-    const Pair N = p_narrow(fma(rwd, wd, -bb)), rt = p_mul(rw, tau), T = p_add(N, rt);
+    const Pair N = p_narrow(fma(rho, w2, -bb)), rt = p_mul(rw, tau), T = p_norm(p_add(N, rt));
     nondeg = !(fabsf(T.h) < 1.0e-30f);
     const Pair x = nondeg ? p_rcp(T) : p_make(0.0f);
     f = p_neg(p_mul(p_mul(bs, tau), x));
@@ -142,7 +149,7 @@ MHDGB_HD bool face_flux_split(const double (&Pl)[NPRIM], const double (&Pr)[NPRI
   const Pair rst = p_sub(ru, r1);
   const Pair fby = p_mul(f, byu), fbz = p_mul(f, bzu), gby = p_mul(g, byu), gbz = p_mul(g, bzu);
   // energy: E* - E = -(tau (E + p_T - rho w S_M) - B_n (v*.B* - v.B)) / w_m, signs as seen from the side
-  Pair es = p_mul(tau, p_sub(p_narrow(ep), p_mul(rw, sms)));
+  Pair es = p_norm(p_mul(tau, p_norm(p_sub(p_narrow(ep), p_mul(rw, sms)))));
   const Pair byst = p_mul(byu, g1), bzst = p_mul(bzu, g1);
   if (!hllc) {
     Pair q = p_mul(bs, tau);
@@ -153,15 +160,15 @@ MHDGB_HD bool face_flux_split(const double (&Pl)[NPRIM], const double (&Pr)[NPRI
     es = p_sub(es, p_mul(bs, q));
     if (!nondeg) es = p_make(0.0f);
   }
-  const Pair S = p_sub(w, vs);                                             // outer wave's speed away from the side
+  const Pair S = p_norm(p_sub(w, vs));                                             // outer wave's speed away from the side
   const Pair am = p_neg_if(S.h > 0.0f ? S : p_make(0.0f), !left);
   const Pair cr = p_mul(r1, am);                                           // corrections to the fluxes
   Pair ce = p_mul(p_mul(es, iwm), am);
   Pair cy = p_mul(am, fby), cz = p_mul(am, fbz), cby = p_mul(am, gby), cbz = p_mul(am, gbz);
   if (!hllc && !(fabsf(bx.h) < 1.0e-30f)) {
     const Pair r1o = p_mul(ro, p_mul(tauo, p_rcp(wmo)));
-    const double rwod = (left ? Pr[nden] : Pl[nden]) * wd;
-    const Pair rto = p_mul(p_narrow_nz(rwod), tauo), To = p_add(p_narrow(fma(rwod, wd, -bb)), rto);
+    const double rhoo = left ? Pr[nden] : Pl[nden];
+    const Pair rto = p_mul(p_mul(ro, w), tauo), To = p_norm(p_add(p_narrow(fma(rhoo, w2, -bb)), rto));
     const bool nondego = !(fabsf(To.h) < 1.0e-30f);
     const Pair xo = nondego ? p_rcp(To) : p_make(0.0f);
     const Pair rsto = nondego ? p_sub(ro, r1o) : ro;
@@ -197,32 +204,32 @@ MHDGB_HD bool face_flux_split(const double (&Pl)[NPRIM], const double (&Pr)[NPRI
   const Pair crx = p_neg_if(p_mul(cr, S), left);                           // (rho* - rho) S, S with its sign
   const Pair cry = p_sub(p_mul(cr, vyu), p_mul(rst, cy)), crz = p_sub(p_mul(cr, vzu), p_mul(rst, cz));
 
-  auto plus = [](double x, Pair c) { return x + p_join(c); };
-  auto minus = [](double x, Pair c) { return x - p_join(c); };
-  const double fr = plus(m, cr);
+  auto wide = [](Pair c) { return p_join(p_norm(c)); };
+  const double fr = m + wide(cr);
   F[mden] = fr;
-  F[mrv1] = plus(fma(m, vx, fma(-bxu, bxu, pt)), crx);
-  F[mrv2] = plus(fma(m, vy, -(by * bxu)), cry);
-  F[mrv3] = plus(fma(m, vz, -(bz * bxu)), crz);
-  F[meto] = plus(fma(ep, vx, -(bsq * bxu)), ce);
-  F[mbm2] = minus(fma(by, vx, -(vy * bxu)), cby);
-  F[mbm3] = minus(fma(bz, vx, -(vz * bxu)), cbz);
-  F[mst] = fr * (left ? Pl[nst] : Pr[nst]);  // the scalar is advected with the mass flux
-  F[mbm1] = 0.5 * fma(-chg, jb, Pl[nbps] + Pr[nbps]);
-  F[mbps] = fma(-hoc, Pr[nbps] - Pl[nbps], hb) * chg2;
-  return true;
+  F[mrv1] = fma(m, vx, fma(-bxu, bxu, pt + wide(crx)));
+  F[mrv2] = fma(m, vy, fma(-by, bxu, wide(cry)));
+  F[mrv3] = fma(m, vz, fma(-bz, bxu, wide(crz)));
+  F[meto] = fma(ep, vx, fma(-bsq, bxu, wide(ce)));
+  F[mbm2] = fma(by, vx, fma(-vy, bxu, wide(p_neg(cby))));
+  F[mbm3] = fma(bz, vx, fma(-vz, bxu, wide(p_neg(cbz))));
+  F[mst] = fr * up(nst, left);  // the scalar is advected with the mass flux
+  F[mbm1] = fma(-hchg, jb, d_half(Pl[nbps] + Pr[nbps]));
+  F[mbps] = fma(-hchg, Pr[nbps] - Pl[nbps], hb * chg2);
+  return ok;
 }
 
 // vanLeer (mhd.cpp:89-95), 2 dp dm / (dp + dm) where the differences have the same sign, from FP64
 // differences: both are scaled by one power of two and taken as pairs, so the slope has the pairs'
 // relative accuracy (about 2^-45) at any magnitude.  Every step is symmetric in dp and dm: the slopes
-// of mirror-image cells are exact mirror images.  Returns false (s untouched) for infinities, NaN and
-// magnitudes below 2^-700, which take the general expression.
-MHDGB_HD bool van_leer_split(double dp, double dm, double& s) {
+// of mirror-image cells are exact mirror images.  ok becomes false for infinities, NaN and
+// magnitudes below 2^-700, which take the general expression; there is no branch, so that a thread's
+// slopes overlap.
+MHDGB_HD double van_leer_split(double dp, double dm, bool& ok) {
   const unsigned hp = d_hi(dp), hm = d_hi(dm), ap = hp & 0x7FFFFFFFu, am = hm & 0x7FFFFFFFu;
   const unsigned top = u_max(ap, am);
   constexpr unsigned lo_lim = (1023u - 700u) << 20, hi_lim = 0x7FF00000u;
-  if (top - lo_lim >= hi_lim - lo_lim) return false;
+  ok = ok && top - lo_lim < hi_lim - lo_lim;
   const unsigned base = (top & 0x7FF00000u) - (127u << 20);  // the larger one scaled into [1, 2)
   // opposite signs, or the smaller one below 2^-71 of the larger: no slope
   const bool flat = (int)(hp ^ hm) < 0 || (int)(u_min(ap, am) - base) < (56 << 20);
@@ -231,32 +238,25 @@ MHDGB_HD bool van_leer_split(double dp, double dm, double& s) {
     return Pair{f_from(f + ((lo >> 28) & 1u)), f_mul(i_to_f((int)(lo << 3)), f_from((f & 0x7F800000u) - (55u << 23)))};
   };
   const Pair x = scaled(ap, d_lo(dp)), y = scaled(am, d_lo(dm));
-  const Pair sum = p_add(x, y);
+  const Pair sum = p_norm(p_add(x, y));
   const float p = f_mul(x.h, y.h);
   const float pl = f_add(f_fma(x.h, y.h, -p), f_fma(x.l, y.l, f_add(f_mul(x.h, y.l), f_mul(x.l, y.h))));
-  const float r = f_rcp_seed(sum.h), q = f_mul(p, r);
+  const float y0 = f_rcp_seed(sum.h), r = f_fma(y0, f_fma(-sum.h, y0, 1.0f), y0), q = f_mul(p, r);
   const float ql = f_mul(r, f_fma(-q, sum.l, f_add(f_fma(-q, sum.h, p), pl)));
-  const double v = p_join(Pair{q, ql}, base - (895u << 20));  // twice the quotient, in the original scale
-  s = flat ? 0.0 : d_from(d_hi(v) | (hp & 0x80000000u), d_lo(v));
-  return true;
+  const double v = p_join(p_norm(Pair{q, ql}), base - (895u << 20));  // twice the quotient, in the original scale
+  return flat ? 0.0 : d_from(d_hi(v) | (hp & 0x80000000u), d_lo(v));
 }
 
 // The cell's candidates for dt (ControlTimestep, mhd.cpp:1542-1550: min over d of dx_d / (|v_d| + sqrt(
 // c_s^2 + B^2/rho))) and c_h (EvaluateCh, mhd.cpp:1589-1601: max over d of |v_d| + c_f,d), which the
-// FP64 form takes at about 2^-43; returns false outside the pairs' range.
+// FP64 form takes at about 2^-43; returns false outside the pairs' range (dt, ch meaningless).
 MHDGB_HD bool cell_speeds_split(const double (&p)[NPRIM], double dx, double dy, double dz, double& dt, double& ch) {
-  {
-    unsigned mx = 0;
+  unsigned mx = u_max(d_mag(p[nden]), d_mag(p[ncsp]));
 #pragma unroll
-    for (int n = 0; n < 3; n++) mx = u_max(mx, u_max(d_mag(p[nve1 + n]), d_mag(p[nbm1 + n])));
-    mx = u_max(mx, u_max(d_mag(p[nden]), d_mag(p[ncsp])));
-    const int mn = (int)kSplitMin;
-    const unsigned smx = u_max(d_mag(dx), u_max(d_mag(dy), d_mag(dz)));
-    const int smn = (int)u_min(d_mag(dx), u_min(d_mag(dy), d_mag(dz)));
-    if (mx >= kSplitMax || (int)d_hi(p[nden]) < mn || (int)d_hi(p[ncsp]) < mn || smx >= kSplitMax ||
-        smn < (int)((1023u - 40u) << 20))
-      return false;
-  }
+  for (int n = 0; n < 3; n++) mx = u_max(mx, u_max(d_mag(p[nve1 + n]), d_mag(p[nbm1 + n])));
+  const unsigned smx = u_max(d_mag(dx), u_max(d_mag(dy), d_mag(dz))), smn = u_min(d_mag(dx), u_min(d_mag(dy), d_mag(dz)));
+  const bool ok = mx < kSplitMax && (int)d_hi(p[nden]) >= (int)kSplitMin && (int)d_hi(p[ncsp]) >= (int)kSplitMin &&
+                  smx < kSplitMax && smn >= (1023u - 40u) << 20;
   const Pair ri = p_rcp(p_narrow_nz(p[nden])), a = p_sqr(p_narrow_nz(p[ncsp]));
   const Pair b1 = p_mul(p_sqr(p_narrow(p[nbm1])), ri), b2 = p_mul(p_sqr(p_narrow(p[nbm2])), ri),
              b3 = p_mul(p_sqr(p_narrow(p[nbm3])), ri);
@@ -266,14 +266,14 @@ MHDGB_HD bool cell_speeds_split(const double (&p)[NPRIM], double dx, double dy, 
   auto time = [ct](double d, Pair v) { return p_mul(p_narrow_nz(d), p_rcp(p_add(v, ct))); };
   const Pair t = p_min(p_min(time(dx, v1), time(dy, v2)), time(dz, v3));
   auto signal = [&](Pair bn, Pair bt, Pair v) {  // |v| + c_f, the discriminant as in face_flux_split
-    const Pair s = p_add(a, bn), d = p_sub(a, bn);
+    const Pair s = p_add(a, bn), d = p_norm(p_sub(a, bn));
     const Pair disc = p_fma(bt, p_add(bt, p_scale(s, 2.0f)), p_sqr(d));
     return p_add(v, p_sqrt(p_scale(p_add(cts, p_sqrt(disc)), 0.5f)));
   };
   const Pair c = p_max(p_max(signal(b1, p_add(b2, b3), v1), signal(b2, p_add(b1, b3), v2)), signal(b3, b12, v3));
-  dt = p_join(t);
-  ch = p_join(c);
-  return true;
+  dt = p_join(p_norm(t));
+  ch = p_join(p_norm(c));
+  return ok;
 }
 
 }  // namespace mhdgb

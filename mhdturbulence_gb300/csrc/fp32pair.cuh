@@ -3,11 +3,11 @@
 //
 // GB300 issues one FP64 warp instruction per SM in about 19 cycles (measured, 16.5 per ns over 152
 // SMs); in that time the four sub-partitions issue up to 76 FP32 or integer instructions, of which
-// the FP64 form used a tenth.  A pair sum takes 11 FP32 instructions and a pair product 7, so moving
+// the FP64 form used a tenth.  A pair sum takes 8 FP32 instructions and a pair product 4, so moving
 // an operation off the FP64 pipe pays five to ten times over.
 //
 // The algorithms are the published error-free transformations (Knuth's TwoSum, Dekker's Fast2Sum,
-// the FMA product of Ogita, Rump and Oishi) and one Newton correction of the hardware's approximate
+// the FMA product of Ogita, Rump and Oishi) and Newton corrections of the hardware's approximate
 // reciprocal and reciprocal square root.  Every operation is rounded to nearest and explicit (no
 // contraction), hence odd in its arguments: mirror-image inputs give mirror-image results.
 #pragma once
@@ -68,7 +68,12 @@ MHDGB_HD int i_clz(unsigned x) { return __builtin_clz(x); }
 MHDGB_HD unsigned f_shl(unsigned hi, unsigned lo, unsigned n) { return n ? (hi << n) | (lo >> (32 - n)) : hi; }
 #endif
 
-// h + l with |l| <= ulp(h)/2 (to a few ulps of l after the cheaper operations).
+// h + l.  The operations leave their results unnormalised: l stays around 2^-23 of the largest term
+// that went into h, but h is not the pair rounded to FP32.  h is then ready one instruction after its
+// operands' h, and the low parts trail behind off the critical path (renormalising after every
+// operation made each wait for the previous one's low part).  Dropped products of low parts are below
+// 2^-46 of the terms.  p_norm() restores |l| <= ulp(h)/2 where terms cancelled and the result is
+// divided by, squared or rooted.
 struct Pair {
   float h, l;
 };
@@ -81,41 +86,32 @@ MHDGB_HD Pair p_neg_if(Pair a, bool n) {
 }
 MHDGB_HD Pair p_sel(bool c, Pair a, Pair b) { return Pair{c ? a.h : b.h, c ? a.l : b.l}; }
 MHDGB_HD Pair p_scale(Pair a, float s) { return Pair{f_mul(a.h, s), f_mul(a.l, s)}; }  // s a power of two
-
-MHDGB_HD Pair two_sum(float a, float b) {
-  const float s = f_add(a, b), v = f_sub(s, a);
-  return Pair{s, f_add(f_sub(a, f_sub(s, v)), f_sub(b, v))};
+MHDGB_HD Pair p_norm(Pair a) {  // |h| >= |l|
+  const float s = f_add(a.h, a.l);
+  return Pair{s, f_sub(a.l, f_sub(s, a.h))};
 }
-MHDGB_HD Pair fast_two_sum(float a, float b) {  // |a| >= |b|
-  const float s = f_add(a, b);
-  return Pair{s, f_sub(b, f_sub(s, a))};
-}
-// a + b with an error of about 2^-47 (|a| + |b|).
+// a + b
 MHDGB_HD Pair p_add(Pair a, Pair b) {
-  const Pair s = two_sum(a.h, b.h);
-  return fast_two_sum(s.h, f_add(s.l, f_add(a.l, b.l)));
+  const float s = f_add(a.h, b.h), v = f_sub(s, a.h);
+  const float e = f_add(f_sub(a.h, f_sub(s, v)), f_sub(b.h, v));
+  return Pair{s, f_add(e, f_add(a.l, b.l))};
 }
 MHDGB_HD Pair p_sub(Pair a, Pair b) { return p_add(a, p_neg(b)); }
 MHDGB_HD Pair p_mul(Pair a, Pair b) {
   const float p = f_mul(a.h, b.h);
-  return fast_two_sum(p, f_fma(a.l, b.h, f_fma(a.h, b.l, f_fma(a.h, b.h, -p))));
+  return Pair{p, f_fma(a.l, b.h, f_fma(a.h, b.l, f_fma(a.h, b.h, -p)))};
 }
 MHDGB_HD Pair p_sqr(Pair a) {
   const float p = f_mul(a.h, a.h);
-  return fast_two_sum(p, f_fma(f_add(a.h, a.h), a.l, f_fma(a.h, a.h, -p)));
+  return Pair{p, f_fma(f_add(a.h, a.h), a.l, f_fma(a.h, a.h, -p))};
 }
 // a * b + c
-MHDGB_HD Pair p_fma(Pair a, Pair b, Pair c) {
-  const float p = f_mul(a.h, b.h);
-  const float e = f_fma(a.l, b.h, f_fma(a.h, b.l, f_fma(a.h, b.h, -p)));
-  const Pair s = two_sum(p, c.h);
-  return fast_two_sum(s.h, f_add(s.l, f_add(e, c.l)));
-}
-// 1 / b: the seed (relative error about 2^-23) is corrected to an FP32 result first, so that the low
-// part is below half an ulp and its own rounding below 2^-48.
+MHDGB_HD Pair p_fma(Pair a, Pair b, Pair c) { return p_add(p_mul(a, b), c); }
+// 1 / b from a seed y: an FP32 reciprocal of h first, then its error against the pair to second order.
 MHDGB_HD Pair p_rcp_from(Pair b, float y) {
   const float r = f_fma(y, f_fma(-b.h, y, 1.0f), y);
-  return fast_two_sum(r, f_mul(r, f_fma(-b.l, r, f_fma(-b.h, r, 1.0f))));
+  const float e = f_fma(-b.l, r, f_fma(-b.h, r, 1.0f));
+  return Pair{r, f_mul(r, f_fma(e, e, e))};
 }
 MHDGB_HD Pair p_rcp(Pair b) { return p_rcp_from(b, f_rcp_seed(b.h)); }
 // sqrt(a) for a >= 0: an FP32 root g and reciprocal root from the seed, then g + (a - g^2) / (2 g)
@@ -126,12 +122,12 @@ MHDGB_HD Pair p_sqrt(Pair a, float* y_out = nullptr) {
   const float y = f_fma(y0, f_fma(-g, y0, 1.0f), y0);
   const float d = f_add(f_fma(-g, g, a.h), a.l);
   if (y_out) *y_out = y;
-  const Pair r = fast_two_sum(g, f_mul(f_mul(0.5f, y), d));
-  return a.h > 0.0f ? r : Pair{0.0f, 0.0f};
+  const bool z = !(a.h > 0.0f);
+  return Pair{z ? 0.0f : g, z ? 0.0f : f_mul(f_mul(0.5f, y), d)};
 }
-MHDGB_HD bool p_less(Pair a, Pair b) { return a.h < b.h || (a.h == b.h && a.l < b.l); }
-MHDGB_HD Pair p_max(Pair a, Pair b) { return p_less(a, b) ? b : a; }
-MHDGB_HD Pair p_min(Pair a, Pair b) { return p_less(b, a) ? b : a; }
+MHDGB_HD bool p_less(Pair a, Pair b) { return f_add(f_sub(a.h, b.h), f_sub(a.l, b.l)) < 0.0f; }
+MHDGB_HD Pair p_max(Pair a, Pair b) { return p_sel(p_less(a, b), b, a); }
+MHDGB_HD Pair p_min(Pair a, Pair b) { return p_sel(p_less(b, a), b, a); }
 
 MHDGB_HD unsigned u_max(unsigned a, unsigned b) { return a > b ? a : b; }
 MHDGB_HD unsigned u_min(unsigned a, unsigned b) { return a < b ? a : b; }
@@ -160,7 +156,12 @@ MHDGB_HD Pair p_narrow(double d) {
   const float l = f_mul(f_mul(i_to_f((int)(lo << 3)), 0x1p-32f), f_from(e | (hi & 0x80000000u)));
   return Pair{z ? 0.0f : d_round_f(hi, lo), z ? 0.0f : l};
 }
-// h + l as a double (within an ulp), on the integer pipe, for |l| <= 2^-22 |h|; ex is added to the
+// x / 2, x zero or normal and above 2^-1021.
+MHDGB_HD double d_half(double x) {
+  const unsigned hi = d_hi(x);
+  return d_from((hi << 1) == 0u ? hi : hi - (1u << 20), d_lo(x));
+}
+// h + l as a double (within an ulp), on the integer pipe, for a normalised pair; ex is added to the
 // result's high word (a power of two, given as its exponent << 20).  h = 0 gives 0.
 MHDGB_HD double p_join(Pair a, unsigned ex = 0u) {
   const unsigned u = f_bits(a.h);

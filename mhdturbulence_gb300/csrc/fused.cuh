@@ -490,8 +490,12 @@ k_fused_step(const InstanceDesc* __restrict__ desc, LaunchCtrl* __restrict__ lc)
     if (kb + 2 <= ke + 1) fill(slot_of(kb + 2));
 
     // work-list sizes and the divisors of their decode
-    const FastDiv dv0(cx), dv1(cx + 1), dv2(cx + 2);
-    const int nxs = cy * (cx + 2), nys = (cy + 2) * cx, nzs = cy * cx;
+    const FastDiv dv0(cx), dv1(cx + 1);
+    // slope items: runs of 6 cells along x and y (the last run of a row starts early enough to end with
+    // it; its overlap is formed twice) for 2 variables, or one cell's 12 variables along z
+    const int ngx = (cx + 7) / 6, ngy = (cy + 7) / 6;
+    const FastDiv dvg(ngx);
+    const int nxs = cy * ngx * 6, nys = ngy * cx * 6, nzs = cy * cx;
     const int nxf = cy * (cx + 1), nyf = (cy + 1) * cx, nzf = cy * cx;
     const int nas = nxs + nys + nzs;
 
@@ -525,40 +529,66 @@ k_fused_step(const InstanceDesc* __restrict__ desc, LaunchCtrl* __restrict__ lc)
         w = __shfl_sync(0xffffffffu, w, 0);
         if (w >= nwa) break;
         const int q = (w << 5) | (tid & 31);
-        if (q < nas) {
-          // one unpadded list over the x, y and z slopes; every direction runs the same loop, whose
-          // code stays small enough for the instruction caches (unrolled over the 12 variables and
-          // three directions the FP64 slopes alone were several times as long)
-          const R *cm, *c0, *cp;  // variable 0 of the cells below, at and above
+        if (q < nxs + nys + nzs) {
+          // 12 slopes a thread, in two batches of 6 that overlap in the pipes: runs of 6 cells along x
+          // or y (neighbours share their differences: 7 subtractions instead of 12) of two variables,
+          // or the 12 variables of a cell along z.  One copy of the arithmetic for all directions keeps
+          // the loop inside the instruction caches.
+          const R *c, *c1 = nullptr, *c2 = nullptr;  // x, y: the run's first cell; z: planes k, k+1, k+2
           R* so;
-          int ostr;
+          int str, ostr, n = 6;
           if (q < nxs) {
-            const int j = dv2.div(q), i = q - j * (cx + 2) - 1;
-            c0 = &PV0(pk, i, j);
-            cm = c0 - 1;
-            cp = c0 + 1;
-            so = &SLX(0, i, j);
-            ostr = TY * (TX + 2);
+            const int r = dvg.div(q), g = q - r * ngx, j = r / 6, v = r - 6 * j, i = max(0, min(6 * g, cx - 4)) - 1;
+            c = &PV0(pk, i, j) + v * PX;
+            so = &SLX(v, i, j);
+            str = ostr = 1;
+            n = cx + 1 - i;
           } else if (q < nxs + nys) {
-            const int r = q - nxs, jr = dv0.div(r), j = jr - 1, i = r - jr * cx;
-            c0 = &PV0(pk, i, j);
-            cm = c0 - NPRIM * PX;
-            cp = c0 + NPRIM * PX;
-            so = &SLY(0, i, j);
-            ostr = (TY + 2) * TX;
+            const int t = q - nxs, r = dv0.div(t), i = t - r * cx, g = r / 6, v = r - 6 * g,
+                      j = max(0, min(6 * g, cy - 4)) - 1;
+            c = &PV0(pk, i, j) + v * PX;
+            so = &SLY(v, i, j);
+            str = NPRIM * PX;
+            ostr = TX;
+            n = cy + 1 - j;
           } else {
             const int r = q - nxs - nys, j = dv0.div(r), i = r - j * cx;
-            cm = &PV0(pk, i, j);
-            c0 = &PV0(pk1, i, j);
-            cp = &PV0(pk2, i, j);
+            c = &PV0(pk, i, j);
+            c1 = &PV0(pk1, i, j);
+            c2 = &PV0(pk2, i, j);
             so = &SLZ(zn, 0, i, j);
+            str = PX;
             ostr = TY * TX;
           }
-          constexpr int UN = kFast && std::is_same<R, double>::value ? 3 : NPRIM;
-#pragma unroll UN
-          for (int n = 0; n < NPRIM; n++) {
-            const R c = c0[n * PX];
-            so[n * ostr] = van_leer(cp[n * PX] - c, c - cm[n * PX]);
+          const int onext = q < nxs ? 6 * TY * (TX + 2) : (q < nxs + nys ? 6 * (TY + 2) * TX : 6 * TY * TX);
+#pragma unroll 1
+          for (int h = 0; h < 2; h++) {
+            R dp[6], dm[6], sl[6];
+            if (c1) {
+#pragma unroll
+              for (int v = 0; v < 6; v++) {
+                const R m = c1[v * PX];
+                dm[v] = m - c[v * PX];
+                dp[v] = c2[v * PX] - m;
+              }
+              c1 += 6 * PX;
+              c2 += 6 * PX;
+            } else {
+              R v = c[-str];
+#pragma unroll
+              for (int m = 0; m < 7; m++) {
+                const R w = c[m * str], d = w - v;
+                if (m < 6) dm[m] = d;
+                if (m > 0) dp[m - 1] = d;
+                v = w;
+              }
+            }
+            c += 6 * PX;
+            van_leer_batch<R, 6>(dp, dm, sl);
+#pragma unroll
+            for (int m = 0; m < 6; m++)
+              if (m < n) so[m * ostr] = sl[m];
+            so += onext;
           }
         }
       }
@@ -622,16 +652,23 @@ k_fused_step(const InstanceDesc* __restrict__ desc, LaunchCtrl* __restrict__ lc)
             return n;
           };
           R pl[NPRIM], pr[NPRIM], f[NCONS];
-#pragma unroll
-          for (int n = 0; n < NPRIM; n++) {
+          auto states = [&](int n) {
             const int v = var_of(n);
             pl[n] = left_state(pa[v * PX], sa[v * sstr]);
             pr[n] = right_state(pb[v * PX], sb[v * sstr]);
-          }
+          };
           if constexpr (kFast && std::is_same<R, double>::value) {
+#pragma unroll
+            for (int n = 0; n < NPRIM; n++)
+              if (n != nene && n != nst) states(n);
+            auto up = [&](int n, bool left) {  // left_state / right_state of the upwind side
+              return fma(left ? 0.5 : -0.5, (left ? sa : sb)[n * sstr], (left ? pa : pb)[n * PX]);
+            };
             if (riemann == RIEMANN_HLLE ||
-                !face_flux_split(pl, pr, glm.chg, glm.hoc, glm.chg2, f, riemann == RIEMANN_HLLC)) {
+                !face_flux_split(pl, pr, up, 0.5 * glm.chg, glm.chg2, f, riemann == RIEMANN_HLLC)) {
               double a[NPRIM], b[NPRIM], c[NCONS];  // copies: only this path puts them in local memory
+              states(nene);
+              states(nst);
 #pragma unroll
               for (int n = 0; n < NPRIM; n++) { a[n] = pl[n]; b[n] = pr[n]; }
               face_flux_general<GEN>(a, b, chg, riemann, rot, c);
@@ -639,6 +676,8 @@ k_fused_step(const InstanceDesc* __restrict__ desc, LaunchCtrl* __restrict__ lc)
               for (int m = 0; m < NCONS; m++) f[m] = c[m];
             }
           } else {
+#pragma unroll
+            for (int n = 0; n < NPRIM; n++) states(n);
             face_flux<R, 0>(pl, pr, glm, f, riemann, rot);
           }
           auto slot_of_flux = [&](int m) {

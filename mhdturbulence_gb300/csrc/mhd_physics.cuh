@@ -224,13 +224,37 @@ __device__ __forceinline__ R van_leer(R dsvp, R dsvm) {
   if constexpr (kFast) {  // one product for the test and the numerator: p + p == (2 dsvp) dsvm exactly
     [[maybe_unused]] const R p = dsvp * dsvm;
     if constexpr (std::is_same<R, double>::value) {
-      double s;
-      return van_leer_split(dsvp, dsvm, s) ? s : van_leer_general(dsvp, dsvm);
+      bool ok = true;
+      const double s = van_leer_split(dsvp, dsvm, ok);
+      return ok ? s : van_leer_general(dsvp, dsvm);
     } else {  // FP32: (p + p) times the MUFU reciprocal, the form the paired evaluation repeats
       return (p > R(0)) ? (p + p) * rcp_approx_f32(dsvp + dsvm) : R(0);
     }
   } else {
     return (dsvp * dsvm > R(0)) ? fdiv(R(2) * dsvp * dsvm, dsvp + dsvm) : R(0);
+  }
+}
+
+// N slopes of a thread, van_leer(dp[n], dm[n]); in the FP64 fast build they overlap, and those the
+// split leaves are replaced afterwards.
+template <class R, int N>
+__device__ __forceinline__ void van_leer_batch(const R (&dp)[N], const R (&dm)[N], R (&s)[N]) {
+  if constexpr (kFast && std::is_same<R, double>::value) {
+    unsigned left = 0;
+#pragma unroll
+    for (int n = 0; n < N; n++) {
+      bool ok = true;
+      s[n] = van_leer_split(dp[n], dm[n], ok);
+      left |= ok ? 0u : 1u << n;
+    }
+    if (left) {
+#pragma unroll
+      for (int n = 0; n < N; n++)
+        if ((left >> n) & 1u) s[n] = van_leer_general(dp[n], dm[n]);
+    }
+  } else {
+#pragma unroll
+    for (int n = 0; n < N; n++) s[n] = van_leer<R>(dp[n], dm[n]);
   }
 }
 
@@ -903,9 +927,14 @@ __device__ __forceinline__ void cons2prim(const R (&u)[NCONS], R gam, R (&p)[NPR
   p[nve1] = u[mrv1] * rhoinv;
   p[nve2] = u[mrv2] * rhoinv;
   p[nve3] = u[mrv3] * rhoinv;
-  const R ekin = R(0.5) * (u[mrv1] * u[mrv1] + u[mrv2] * u[mrv2] + u[mrv3] * u[mrv3]) * rhoinv;
-  const R emag = R(0.5) * (u[mbm1] * u[mbm1] + u[mbm2] * u[mbm2] + u[mbm3] * u[mbm3]);
-  p[nene] = kFast ? (u[meto] - ekin - emag) * rhoinv : (u[meto] - ekin - emag) / u[mden];
+  const R m2 = u[mrv1] * u[mrv1] + u[mrv2] * u[mrv2] + u[mrv3] * u[mrv3];
+  const R b2 = u[mbm1] * u[mbm1] + u[mbm2] * u[mbm2] + u[mbm3] * u[mbm3];
+  if constexpr (kFast) {  // (E - m^2 / (2 rho) - B^2 / 2) / rho in two FMAs
+    p[nene] = fma(R(-0.5) * rhoinv, m2, fma(R(-0.5), b2, u[meto])) * rhoinv;
+  } else {
+    const R ekin = R(0.5) * m2 * rhoinv, emag = R(0.5) * b2;
+    p[nene] = (u[meto] - ekin - emag) / u[mden];
+  }
   p[npre] = p[nene] * p[nden] * (gam - R(1));
   p[ncsp] = fsqrt_est(p[nene] * gam * (gam - R(1)));  // the sound speed only enters wave-speed estimates
   p[nbm1] = u[mbm1];
