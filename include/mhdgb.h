@@ -213,7 +213,9 @@ int mhdgb_measure_fp64_rate(int device, double* gflops);
 /* Self-test of the FP64 division and square root used by the FMA-contracted FP64 form (FP32-seeded
  * reciprocal with two Newton-Raphson steps; FP32-seeded Goldschmidt square root and reciprocal
  * square root) against IEEE division and square root on n random operands; *max_ulp receives the
- * largest difference in units in the last place. */
+ * largest difference in units in the last place.  The separately rounded kernels' division and square
+ * root (integer remainders) are checked along with them, also on operands of any exponent, and have to
+ * equal IEEE's: a difference there counts as 2^20 units. */
 int mhdgb_selftest_division(int device, int n, unsigned long long seed, double* max_ulp);
 /* Self-test of failure detection (no reference counterpart): a kernel waits on a shared-memory
  * barrier that nothing completes; the bounded wait the fused step uses for its plane loads gives

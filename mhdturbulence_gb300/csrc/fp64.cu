@@ -8,8 +8,8 @@
 namespace mhdgb {
 namespace {
 
-// The FP64 division, square root and reciprocal square root of the fast build against IEEE
-// division and square root on log-uniform operands (both signs for the division) over
+// The FP64 division, square root and reciprocal square root of the fast build, and the correctly
+// rounded ones of the exact build, against IEEE division and square root on log-uniform operands (both signs for the division) over
 // [2^-60, 2^60]: the largest distance in units in the last place.
 __global__ void k_fdiv_selftest(int n, unsigned long long seed, unsigned long long* max_ulp) {
   unsigned long long worst = 0;
@@ -37,6 +37,16 @@ __global__ void k_fdiv_selftest(int n, unsigned long long seed, unsigned long lo
     const unsigned long long adi = (unsigned long long)(di < 0 ? -di : di);
     if (ads > worst) worst = ads;
     if (adi > worst) worst = adi;
+    // the correctly rounded division and root of the exact build, on operands of any exponent (zero,
+    // subnormal, infinite and NaN among them) and on nearly equal significands: any difference counts
+    // as 2^20 ulp
+    const unsigned long long bu = next(), bv = (t & 3) ? next() : (bu ^ (next() & 0x7FF0000000000007ull));
+    const double eu = __longlong_as_double((long long)bu), ev = __longlong_as_double((long long)bv);
+    const double eq = div_rn(eu, ev), es = sqrt_rn(eu);
+    auto differ = [](double x, double y) {
+      return __double_as_longlong(x) != __double_as_longlong(y) && !(x != x && y != y);
+    };
+    if (differ(eq, eu / ev) || differ(es, sqrt(eu)) || differ(div_rn(a, b), r) || differ(sqrt_rn(x), sr)) worst = 1ull << 20;
   }
   atomicMax(max_ulp, worst);
 }

@@ -278,7 +278,7 @@ __device__ __forceinline__ void update_cell(const DivAcc<double>& acc, const dou
     double dhl = a.dxs[i];
     if (a.dys[j] < dhl) dhl = a.dys[j];
     if (a.dzs[k] < dhl) dhl = a.dzs[k];
-    const double taui = 0.1 * chd / dhl;
+    const double taui = fdiv(0.1 * chd, dhl);
     u[mbps] = u[mbps] * (1.0 - dt * taui);
   }
 }

@@ -22,6 +22,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "exact64.cuh"
 #include "face_split.cuh"
 
 namespace mhdgb {
@@ -130,11 +131,14 @@ __device__ __forceinline__ double sqrt_goldschmidt(double x, double* inv = nullp
   return fma(d, h, g);
 }
 
-// sqrt: IEEE in the exact build and in FP32; sqrt_goldschmidt in the FP64 fast build.
+// sqrt: correctly rounded in the exact build, off the FP64 pipe (sqrt_rn); the build's sqrt in FP32;
+// sqrt_goldschmidt in the FP64 fast build.
 template <class R>
 __device__ __forceinline__ R fsqrt(R x) {
   if constexpr (kFast && std::is_same<R, double>::value) {
     return sqrt_seed_range(x) ? sqrt_goldschmidt(x) : sqrt(x);
+  } else if constexpr (std::is_same<R, double>::value) {
+    return sqrt_rn(x);
   } else {
     return sqrt(x);
   }
@@ -159,11 +163,11 @@ __device__ __forceinline__ R fsqrt_est(R x) {
     const double d = fma(-g0d, g0d, x);
     return g0d + f2d_exact(d2f_rne(d) * (0.5f * yf));
   } else {
-    return sqrt(x);
+    return fsqrt(x);
   }
 }
 
-// a / b: IEEE division in the exact build; a * rcp_newton(b) in the FP64 fast build (within ~1.5
+// a / b: correctly rounded in the exact build, off the FP64 pipe (div_rn); a * rcp_newton(b) in the FP64 fast build (within ~1.5
 // ulp), with IEEE division where |b| is outside the FP32 seed's range; in the FP32 (mixed) build a
 // times the MUFU reciprocal (within ~2 ulp, like the build's approximate division, with fewer
 // instructions).
@@ -176,7 +180,7 @@ __device__ __forceinline__ R fdiv(R a, R b) {
   } else if constexpr (kFast && std::is_same<R, float>::value) {
     return a * rcp_approx_f32(b);
   } else {
-    return a / b;
+    return div_rn(a, b);
   }
 }
 
@@ -197,6 +201,30 @@ __device__ __forceinline__ R fdiv_est(R a, R b) {
     return fdiv(a, b);
   }
 }
+
+// x / 2, and min / max with the reference's std::min / std::max results, for the exact build on the
+// integer pipe.
+template <class R>
+__device__ __forceinline__ R half_of(R x) {
+  if constexpr (!kFast && std::is_same<R, double>::value) {
+    const unsigned hi = d_hi(x), lo = d_lo(x), e = (hi >> 20) & 0x7FFu;
+    if (e - 2u < 2045u) return d_from(hi - (1u << 20), lo);
+    if (((hi << 1) | lo) == 0u) return x;
+  }
+  return R(0.5) * x;
+}
+template <class R>
+__device__ __forceinline__ bool less_than(R a, R b) {
+  if constexpr (!kFast && std::is_same<R, double>::value) {  // a < b: zeros of either sign equal, NaN never less
+    const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+    constexpr long long mag = 0x7FFFFFFFFFFFFFFFLL, inf = 0x7FF0000000000000LL;
+    return order_key(a) < order_key(b) && ((x | y) & mag) != 0 && (x & mag) <= inf && (y & mag) <= inf;
+  } else {
+    return a < b;
+  }
+}
+template <class R> __device__ __forceinline__ R xmin(R a, R b) { return less_than(b, a) ? b : a; }
+template <class R> __device__ __forceinline__ R xmax(R a, R b) { return less_than(a, b) ? b : a; }
 
 // 2p / s at the accuracy of fdiv_est, with the factor 2 taken into the FP32 seed (exact there):
 // y0 = 2 r0 and one Newton step y1 = y0 + r0 (2 - s y0) = 2 r0 (2 - s r0).  One FP64 operation fewer
@@ -231,7 +259,10 @@ __device__ __forceinline__ R van_leer(R dsvp, R dsvm) {
       return (p > R(0)) ? (p + p) * rcp_approx_f32(dsvp + dsvm) : R(0);
     }
   } else {
-    return (dsvp * dsvm > R(0)) ? fdiv(R(2) * dsvp * dsvm, dsvp + dsvm) : R(0);
+    const R p = dsvp * dsvm;
+    if (!pos_nonzero(p)) return R(0);
+    const unsigned e = (unsigned)__double2hiint(p) >> 20;  // 2 dsvp dsvm is 2 p unless p is subnormal
+    return fdiv(e - 1u < 2045u ? d_from(d_hi(p) + (1u << 20), d_lo(p)) : R(2) * dsvp * dsvm, dsvp + dsvm);
   }
 }
 
@@ -338,13 +369,13 @@ __device__ __forceinline__ void prim2cons(const R (&Prim)[NPRIM], R (&Cons)[NVEC
   Cons[D::muv1] = rho * Prim[nve1];
   Cons[D::muv2] = rho * Prim[nve2];
   Cons[D::muv3] = rho * Prim[nve3];
-  Cons[muet] = rho * Prim[nene] + R(0.5) * rho * vsq + R(0.5) * bsq;
+  Cons[muet] = rho * Prim[nene] + half_of(rho) * vsq + half_of(bsq);
   Cons[D::mub1] = Prim[nbm1];
   Cons[D::mub2] = Prim[nbm2];
   Cons[D::mub3] = Prim[nbm3];
   Cons[mubp] = Prim[nbps];
   Cons[must] = rho * Prim[nst];
-  const R ptl = Prim[npre] + bsq / R(2);
+  const R ptl = Prim[npre] + half_of(bsq);
   Cons[mfdn] = rho * Prim[D::nved];
   Cons[D::mfv1] = rho * Prim[nve1] * Prim[D::nved] - Prim[nbm1] * Prim[D::nbmd];
   Cons[D::mfv2] = rho * Prim[nve2] * Prim[D::nved] - Prim[nbm2] * Prim[D::nbmd];
@@ -358,7 +389,7 @@ __device__ __forceinline__ void prim2cons(const R (&Prim)[NPRIM], R (&Cons)[NVEC
   Cons[mfst] = rho * Prim[nst] * Prim[D::nved];
   const R css = Prim[ncsp] * Prim[ncsp];
   const R cts = css + bsq * rhoinv;
-  Cons[mcsp] = fsqrt_est((cts + fsqrt_est(cts * cts - R(4) * css * Prim[D::nbmd] * Prim[D::nbmd] * rhoinv)) / R(2));
+  Cons[mcsp] = fsqrt_est(half_of(cts + fsqrt_est(cts * cts - R(4) * css * Prim[D::nbmd] * Prim[D::nbmd] * rhoinv)));
   Cons[mvel] = Prim[D::nved];
   Cons[mpre] = ptl;
 }
@@ -377,7 +408,7 @@ __device__ __forceinline__ void prim2cons_state(const R (&Prim)[NPRIM], R (&Cons
   Cons[D::muv1] = rho * Prim[nve1];
   Cons[D::muv2] = rho * Prim[nve2];
   Cons[D::muv3] = rho * Prim[nve3];
-  Cons[muet] = rho * Prim[nene] + R(0.5) * rho * vsq + R(0.5) * bsq;
+  Cons[muet] = rho * Prim[nene] + half_of(rho) * vsq + half_of(bsq);
   Cons[D::mub1] = Prim[nbm1];
   Cons[D::mub2] = Prim[nbm2];
   Cons[D::mub3] = Prim[nbm3];
@@ -385,9 +416,9 @@ __device__ __forceinline__ void prim2cons_state(const R (&Prim)[NPRIM], R (&Cons
   Cons[must] = rho * Prim[nst];
   const R css = Prim[ncsp] * Prim[ncsp];
   const R cts = css + bsq * rhoinv;
-  Cons[mcsp] = fsqrt_est((cts + fsqrt_est(cts * cts - R(4) * css * Prim[D::nbmd] * Prim[D::nbmd] * rhoinv)) / R(2));
+  Cons[mcsp] = fsqrt_est(half_of(cts + fsqrt_est(cts * cts - R(4) * css * Prim[D::nbmd] * Prim[D::nbmd] * rhoinv)));
   Cons[mvel] = Prim[D::nved];
-  Cons[mpre] = Prim[npre] + bsq / R(2);
+  Cons[mpre] = Prim[npre] + half_of(bsq);
 }
 // The left (x) and right (y) lanes of packed state pairs, indexed like a state vector.
 struct PairLo {
@@ -451,155 +482,111 @@ __device__ __forceinline__ void prim2cons_flux(const R (&Prim)[NPRIM], R (&Cons)
   Cons[mfst] = rho * Prim[nst] * Prim[D::nved];
 }
 
-// HLLD, mhd.cpp:97-417.  Writes the 10 rotated fluxes (slot mubp is left undefined: the GLM pair
-// replaces it).
-// Fast forms: the velocities m/rho of the rotated states are the reconstructed primitive
-// velocities themselves (Cons[muv?] = rho * Prim[nve?]), and rho*X/rho is X.
-template <class R, int DIR>
-__device__ __forceinline__ void hlld(const R (&leftst)[NVEC], const R (&rigtst)[NVEC], const R (&Pl)[NPRIM],
-                                     const R (&Pr)[NPRIM], R (&nflux)[NCONS]) {
-  using D = Dir<DIR>;
-  const R eps = R(1.0e-30);
-  const R rol = leftst[mudn], eel = leftst[muet];
-  const R rxl = leftst[muvu], ryl = leftst[muvv], rzl = leftst[muvw];
-  const R vxl = kFast ? Pl[D::nved] : leftst[muvu] / leftst[mudn];
-  const R vyl = kFast ? Pl[D::nvef] : leftst[muvv] / leftst[mudn];
-  const R vzl = kFast ? Pl[D::nveb] : leftst[muvw] / leftst[mudn];
-  const R byl = leftst[mubv], bzl = leftst[mubw], ptl = leftst[mpre], scl = leftst[must];
-  const R ror = rigtst[mudn], eer = rigtst[muet];
-  const R rxr = rigtst[muvu], ryr = rigtst[muvv], rzr = rigtst[muvw];
-  const R vxr = kFast ? Pr[D::nved] : rigtst[muvu] / rigtst[mudn];
-  const R vyr = kFast ? Pr[D::nvef] : rigtst[muvv] / rigtst[mudn];
-  const R vzr = kFast ? Pr[D::nveb] : rigtst[muvw] / rigtst[mudn];
-  const R byr = rigtst[mubv], bzr = rigtst[mubw], ptr = rigtst[mpre], scr = rigtst[must];
-
+// HLLD, mhd.cpp:97-417, for the exact build: the reference's expressions, operation by operation, with
+// its 0/1 masks (maxs1 / mins1 of mhd.cpp:272-275, 306-308, 343-346, 384-386) taken as selections, which
+// leaves every finite result the same (a product with a mask and the sum with the masked-out zero are
+// exact), and the flux formed for the upwind side only (prim2cons_flux fills its flux slots).  Divisions,
+// roots, comparisons and halvings run off the FP64 pipe, which bounds this build.  Writes the 10
+// rotated fluxes (slot mubp is left undefined: the GLM pair replaces it).
+template <int DIR>
+__device__ __forceinline__ void hlld(const double (&leftst)[NVEC], const double (&rigtst)[NVEC],
+                                     const double (&Pl)[NPRIM], const double (&Pr)[NPRIM], double (&nflux)[NCONS],
+                                     int rot = 0) {
+  using R = double;
+  const R eps = 1.0e-30;
+  const R vxl = fdiv(leftst[muvu], leftst[mudn]), vyl = fdiv(leftst[muvv], leftst[mudn]),
+          vzl = fdiv(leftst[muvw], leftst[mudn]);
+  const R vxr = fdiv(rigtst[muvu], rigtst[mudn]), vyr = fdiv(rigtst[muvv], rigtst[mudn]),
+          vzr = fdiv(rigtst[muvw], rigtst[mudn]);
+  const R ptl = leftst[mpre], ptr = rigtst[mpre];
   // Step 1 (mhd.cpp:212-216)
-  const R cfl = leftst[mcsp], cfr = rigtst[mcsp];
-  const R sl = smin(vxl, vxr) - smax(cfl, cfr);
-  const R sr = smax(vxl, vxr) + smax(cfl, cfr);
-  // Step 2 (mhd.cpp:221-243)
-  const R frol = leftst[mfdn], feel = leftst[mfet], frxl = leftst[mfvu], fryl = leftst[mfvv];
-  const R frzl = leftst[mfvw], fbyl = leftst[mfbv], fbzl = leftst[mfbw], fscl = leftst[mfst];
-  const R fror = rigtst[mfdn], feer = rigtst[mfet], frxr = rigtst[mfvu], fryr = rigtst[mfvv];
-  const R frzr = rigtst[mfvw], fbyr = rigtst[mfbv], fbzr = rigtst[mfbw], fscr = rigtst[mfst];
+  const R cfast = xmax(leftst[mcsp], rigtst[mcsp]);
+  const R sl = xmin(vxl, vxr) - cfast, sr = xmax(vxl, vxr) + cfast;
   // Step 4 (mhd.cpp:248-258)
-  const R sdl = smin(R(-1e-20), sl - vxl);
-  const R sdr = smax(R(1e-20), sr - vxr);
-  const R rosdl = rol * sdl;
-  const R rosdr = ror * sdr;
-  R temp = fdiv(R(1), rosdr - rosdl);
-  const R sm = (rosdr * vxr - rosdl * vxl - ptr + ptl) * temp;
-  const R sdml = smin(R(-1e-20), sl - sm);
-  const R isdml = fdiv(R(1), sdml);
-  const R sdmr = smax(R(1e-20), sr - sm);
-  const R isdmr = fdiv(R(1), sdmr);
+  const R sdl = xmin(-1e-20, sl - vxl), sdr = xmax(1e-20, sr - vxr);
+  const R rosdl = leftst[mudn] * sdl, rosdr = rigtst[mudn] * sdr;
+  const R tden = fdiv(1.0, rosdr - rosdl);
+  const R sm = (rosdr * vxr - rosdl * vxl - ptr + ptl) * tden;
+  const R sdml = xmin(-1e-20, sl - sm), sdmr = xmax(1e-20, sr - sm);
   // Step 5 (mhd.cpp:264)
-  const R ptst = (rosdr * ptl - rosdl * ptr + rosdl * rosdr * (vxr - vxl)) * temp;
-  // Step 5A (mhd.cpp:269-300)
-  const R bxs = R(0.5) * (leftst[mubu] + rigtst[mubu]);
+  const R ptst = (rosdr * ptl - rosdl * ptr + rosdl * rosdr * (vxr - vxl)) * tden;
+  const R bxs = half_of(leftst[mubu] + rigtst[mubu]);
   const R bxsq = bxs * bxs;
-  // Degenerate star states (rho (S - v)(S - S_M) = B_x^2, e.g. field-aligned flow with c_f = v_A):
-  // the reference switches to v* = v, B* = B below |T| < 1e-30, which FP64 rounding noise (~1e-16)
-  // never reaches.  In FP32, T and the numerators it divides are rounding noise (~1e-7 of p_T*)
-  // near degeneracy, so the FP32 solver treats |T| < 1e-6 p_T* (about eight FP32 ulps of the star
-  // total pressure) as degenerate.  Above that the FP32 star state still follows FP64's: on the
-  // low-beta KH layer (B_x = 1, p = 0.1) thresholds from 3e-7 to 3e-6 give the same state, while
-  // 1e-5 and above switch faces the FP64 solver resolves, and its absolute 1e-30 fails in FP32.
-  const R deg = std::is_same<R, float>::value ? smax(eps, R(1e-6) * fabs(ptst)) : eps;
-  R temp_fst = rosdl * sdml - bxsq;
-  R sign1 = copysign(R(1), fabs(temp_fst) - deg);
-  R maxs1 = smax(R(0), sign1);
-  R mins1 = smin(R(0), sign1);
-  R itf = fdiv(R(1), temp_fst + mins1);
-  temp = bxs * (sdl - sdml) * itf;
-  const R rolst = maxs1 * (rosdl * isdml) - mins1 * rol;
-  const R sclst = kFast ? rolst * Pl[nst] : rolst / rol * scl;
-  const R vxlst = maxs1 * sm - mins1 * vxl;
-  const R rxlst = rolst * vxlst;
-  const R vylst = maxs1 * (vyl - byl * temp) - mins1 * vyl;
-  const R rylst = rolst * vylst;
-  const R vzlst = maxs1 * (vzl - bzl * temp) - mins1 * vzl;
-  const R rzlst = rolst * vzlst;
-  temp = (rosdl * sdl - bxsq) * itf;
-  const R bylst = maxs1 * (byl * temp) - mins1 * byl;
-  const R bzlst = maxs1 * (bzl * temp) - mins1 * bzl;
-  const R vdbstl = vxlst * bxs + vylst * bylst + vzlst * bzlst;
-  const R eelst = maxs1 * (sdl * eel - ptl * vxl + ptst * sm +
-                           bxs * (vxl * bxs + vyl * byl + vzl * bzl - vdbstl)) * isdml
-                  - mins1 * eel;
-  // Step 5B (mhd.cpp:305-333)
-  temp_fst = rosdr * sdmr - bxsq;
-  sign1 = copysign(R(1), fabs(temp_fst) - deg);
-  maxs1 = smax(R(0), sign1);
-  mins1 = smin(R(0), sign1);
-  itf = fdiv(R(1), temp_fst + mins1);
-  temp = bxs * (sdr - sdmr) * itf;
-  const R rorst = maxs1 * (rosdr * isdmr) - mins1 * ror;
-  const R scrst = kFast ? rorst * Pr[nst] : rorst / ror * scr;
-  const R vxrst = maxs1 * sm - mins1 * vxr;
-  const R rxrst = rorst * vxrst;
-  const R vyrst = maxs1 * (vyr - byr * temp) - mins1 * vyr;
-  const R ryrst = rorst * vyrst;
-  const R vzrst = maxs1 * (vzr - bzr * temp) - mins1 * vzr;
-  const R rzrst = rorst * vzrst;
-  temp = (rosdr * sdr - bxsq) * itf;
-  const R byrst = maxs1 * (byr * temp) - mins1 * byr;
-  const R bzrst = maxs1 * (bzr * temp) - mins1 * bzr;
-  const R vdbstr = vxrst * bxs + vyrst * byrst + vzrst * bzrst;
-  const R eerst = maxs1 * ((sdr * eer - ptr * vxr + ptst * sm) * isdmr +
-                           bxs * (vxr * bxs + vyr * byr + vzr * bzr - vdbstr) * isdmr)
-                  - mins1 * eer;
-  // Step 5C (mhd.cpp:338-377)
-  const R sqrtrol = sqrt(rolst);
-  const R sqrtror = sqrt(rorst);
-  const R abbx = fabs(bxs);
-  const R signbx = copysign(R(1), bxs);
-  sign1 = copysign(R(1), abbx - eps);
-  maxs1 = smax(R(0), sign1);
-  mins1 = -smin(R(0), sign1);
-  const R invsumro = fdiv(maxs1, sqrtrol + sqrtror);
-  temp = invsumro * (sqrtrol * vylst + sqrtror * vyrst + signbx * (byrst - bylst));
-  const R vyldst = vylst * mins1 + temp;
-  const R ryldst = rylst * mins1 + rolst * temp;
-  const R ryrdst = ryrst * mins1 + rorst * temp;
-  temp = invsumro * (sqrtrol * vzlst + sqrtror * vzrst + signbx * (bzrst - bzlst));
-  const R vzldst = vzlst * mins1 + temp;
-  const R rzldst = rzlst * mins1 + rolst * temp;
-  const R rzrdst = rzrst * mins1 + rorst * temp;
-  temp = invsumro * (sqrtrol * byrst + sqrtror * bylst + signbx * sqrtrol * sqrtror * (vyrst - vylst));
-  const R byldst = bylst * mins1 + temp;
-  const R byrdst = byrst * mins1 + temp;
-  temp = invsumro * (sqrtrol * bzrst + sqrtror * bzlst + signbx * sqrtrol * sqrtror * (vzrst - vzlst));
-  const R bzldst = bzlst * mins1 + temp;
-  const R bzrdst = bzrst * mins1 + temp;
-  temp = sm * bxs + vyldst * byldst + vzldst * bzldst;
-  const R eeldst = eelst - sqrtrol * signbx * (vdbstl - temp) * maxs1;
-  const R eerdst = eerst + sqrtror * signbx * (vdbstr - temp) * maxs1;
-  // Step 6 (mhd.cpp:381-415)
-  const R slst = (sm - fdiv(abbx, sqrtrol)) * maxs1;
-  const R srst = (sm + fdiv(abbx, sqrtror)) * maxs1;
-  sign1 = copysign(R(1), sm);
-  maxs1 = smax(R(0), sign1);
-  mins1 = -smin(R(0), sign1);
-  const R msl = smin(sl, R(0));
-  const R msr = smax(sr, R(0));
-  const R mslst = smin(slst, R(0));
-  const R msrst = smax(srst, R(0));
-  nflux[mden] = (frol + (rolst - rol) * msl) * maxs1 + (fror + (rorst - ror) * msr) * mins1;
-  nflux[meto] = (feel + (eelst - eel) * msl + (eeldst - eelst) * mslst) * maxs1
-              + (feer + (eerst - eer) * msr + (eerdst - eerst) * msrst) * mins1;
-  nflux[mrv1] = (frxl + (rxlst - rxl) * msl) * maxs1 + (frxr + (rxrst - rxr) * msr) * mins1;
-  nflux[mrv2] = (fryl + (rylst - ryl) * msl + (ryldst - rylst) * mslst) * maxs1
-              + (fryr + (ryrst - ryr) * msr + (ryrdst - ryrst) * msrst) * mins1;
-  nflux[mrv3] = (frzl + (rzlst - rzl) * msl + (rzldst - rzlst) * mslst) * maxs1
-              + (frzr + (rzrst - rzr) * msr + (rzrdst - rzrst) * msrst) * mins1;
-  nflux[mbm1] = R(0);
-  nflux[mbm2] = (fbyl + (bylst - byl) * msl + (byldst - bylst) * mslst) * maxs1
-              + (fbyr + (byrst - byr) * msr + (byrdst - byrst) * msrst) * mins1;
-  nflux[mbm3] = (fbzl + (bzlst - bzl) * msl + (bzldst - bzlst) * mslst) * maxs1
-              + (fbzr + (bzrst - bzr) * msr + (bzrdst - bzrst) * msrst) * mins1;
-  nflux[mst] = (fscl + (sclst - scl) * msl) * maxs1 + (fscr + (scrst - scr) * msr) * mins1;
-  nflux[mbps] = R(0);
+  const bool left = !signbit(sm);
+  // star states of the upwind side (u) and the other (o), Steps 5A and 5B (mhd.cpp:269-333)
+  struct Star {
+    R ro, vx, vy, vz, by, bz, isdm;
+    bool nondeg;
+  };
+  auto star = [&](R ro, R vx, R vy, R vz, R by, R bz, R sd, R rosd, R sdm) {
+    Star t;
+    t.isdm = fdiv(1.0, sdm);
+    const R f = rosd * sdm - bxsq;
+    t.nondeg = !abs_less(f, eps);
+    const R itf = fdiv(1.0, f);
+    const R t1 = bxs * (sd - sdm) * itf, t2 = (rosd * sd - bxsq) * itf;
+    t.ro = t.nondeg ? rosd * t.isdm : ro;
+    t.vx = t.nondeg ? sm : vx;
+    t.vy = t.nondeg ? vy - by * t1 : vy;
+    t.vz = t.nondeg ? vz - bz * t1 : vz;
+    t.by = t.nondeg ? by * t2 : by;
+    t.bz = t.nondeg ? bz * t2 : bz;
+    return t;
+  };
+  auto sel = [left](R a, R b) { return left ? a : b; };
+  R cst[NVEC], pup[NPRIM];  // the upwind side's vectors
+#pragma unroll
+  for (int q = 0; q < NVEC; q++) cst[q] = sel(leftst[q], rigtst[q]);
+#pragma unroll
+  for (int n = 0; n < NPRIM; n++) pup[n] = sel(Pl[n], Pr[n]);
+  const R ro = cst[mudn], by = cst[mubv], bz = cst[mubw], ee = cst[muet], pt = cst[mpre];
+  const R vx = sel(vxl, vxr), vy = sel(vyl, vyr), vz = sel(vzl, vzr), sd = sel(sdl, sdr);
+  const Star u = star(ro, vx, vy, vz, by, bz, sd, sel(rosdl, rosdr), sel(sdml, sdmr));
+  const Star o = star(sel(rigtst[mudn], leftst[mudn]), sel(vxr, vxl), sel(vyr, vyl), sel(vzr, vzl),
+                      sel(rigtst[mubv], leftst[mubv]), sel(rigtst[mubw], leftst[mubw]), sel(sdr, sdl),
+                      sel(rosdr, rosdl), sel(sdmr, sdml));
+  const R rost = u.ro, rxst = rost * u.vx, ryst = rost * u.vy, rzst = rost * u.vz;
+  const R vdbst = u.vx * bxs + u.vy * u.by + u.vz * u.bz;
+  R eest = ee;
+  if (u.nondeg) {  // the reference sums the two sides' numerators in different orders (mhd.cpp:297-300, 329-333)
+    const R a = sd * ee - pt * vx + ptst * sm, b = bxs * (vx * bxs + vy * by + vz * bz - vdbst);
+    eest = left ? (a + b) * u.isdm : a * u.isdm + b * u.isdm;
+  }
+  // Step 5C (mhd.cpp:338-377) and the Alfven speed of Step 6 (mhd.cpp:381-383)
+  R rydst = ryst, rzdst = rzst, bydst = u.by, bzdst = u.bz, eedst = eest, sst = 0.0;
+  if (!abs_less(bxs, eps)) {
+    const R sq = fsqrt(rost), sqo = fsqrt(o.ro);
+    const R ql = sel(sq, sqo), qr = sel(sqo, sq);
+    const R vylst = sel(u.vy, o.vy), vyrst = sel(o.vy, u.vy), vzlst = sel(u.vz, o.vz), vzrst = sel(o.vz, u.vz);
+    const R bylst = sel(u.by, o.by), byrst = sel(o.by, u.by), bzlst = sel(u.bz, o.bz), bzrst = sel(o.bz, u.bz);
+    const bool neg = signbit(bxs);
+    const R inv = fdiv(1.0, ql + qr);
+    const R vydst = inv * (ql * vylst + qr * vyrst + negate_if(byrst - bylst, neg));
+    const R vzdst = inv * (ql * vzlst + qr * vzrst + negate_if(bzrst - bzlst, neg));
+    const R sqq = negate_if(ql, neg) * qr;
+    bydst = inv * (ql * byrst + qr * bylst + sqq * (vyrst - vylst));
+    bzdst = inv * (ql * bzrst + qr * bzlst + sqq * (vzrst - vzlst));
+    rydst = rost * vydst;
+    rzdst = rost * vzdst;
+    const R vdb = sm * bxs + vydst * bydst + vzdst * bzdst;
+    const R de = negate_if(sq, neg) * (vdbst - vdb);
+    eedst = left ? eest - de : eest + de;
+    const R sa = fdiv(fabs(bxs), sq);
+    sst = left ? sm - sa : sm + sa;
+  }
+  // Step 6 (mhd.cpp:384-415)
+  const R ms = left ? xmin(sl, 0.0) : xmax(sr, 0.0), msst = left ? xmin(sst, 0.0) : xmax(sst, 0.0);
+  prim2cons_flux<R, DIR>(pup, cst, rot);
+  nflux[mden] = cst[mfdn] + (rost - ro) * ms;
+  nflux[meto] = cst[mfet] + (eest - ee) * ms + (eedst - eest) * msst;
+  nflux[mrv1] = cst[mfvu] + (rxst - cst[muvu]) * ms;
+  nflux[mrv2] = cst[mfvv] + (ryst - cst[muvv]) * ms + (rydst - ryst) * msst;
+  nflux[mrv3] = cst[mfvw] + (rzst - cst[muvw]) * ms + (rzdst - rzst) * msst;
+  nflux[mbm1] = 0.0;
+  nflux[mbm2] = cst[mfbv] + (u.by - by) * ms + (bydst - u.by) * msst;
+  nflux[mbm3] = cst[mfbw] + (u.bz - bz) * ms + (bzdst - u.bz) * msst;
+  nflux[mst] = cst[mfst] + (fdiv(rost, ro) * cst[must] - cst[must]) * ms;
+  nflux[mbps] = 0.0;
 }
 
 // HLLD in branch form, for the FMA-contracted builds (FP64 and the mixed form's FP32 solve).  Same
@@ -656,7 +643,13 @@ __device__ __forceinline__ void hlld_branch(const CL& leftst, const CR& rigtst, 
   // star state of the upwind side (Step 5A/5B); one reciprocal of sdm * T gives 1/sdm and 1/T
   R rost = ro, vxst = vx, vyst = vy, vzst = vz, byst = by, bzst = bz;
   const R temp_fst = rosd * sdm - bxsq;
-  // FP32: the degenerate-state guard relative to the star total pressure (see hlld())
+  // Degenerate star states (rho (S - v)(S - S_M) = B_x^2, e.g. field-aligned flow with c_f = v_A):
+  // the reference switches to v* = v, B* = B below |T| < 1e-30, which FP64 rounding noise (~1e-16)
+  // never reaches.  In FP32, T and the numerators it divides are rounding noise (~1e-7 of p_T*)
+  // near degeneracy, so the FP32 solver treats |T| < 1e-6 p_T* (about eight FP32 ulps of the star
+  // total pressure) as degenerate.  Above that the FP32 star state still follows FP64's: on the
+  // low-beta KH layer (B_x = 1, p = 0.1) thresholds from 3e-7 to 3e-6 give the same state, while
+  // 1e-5 and above switch faces the FP64 solver resolves, and its absolute 1e-30 fails in FP32.
   const R deg = std::is_same<R, float>::value ? imax(eps, R(1e-6) * fabs(ptst)) : eps;
   const bool nondeg = !abs_less(temp_fst, deg);
   R isdm = R(0);
@@ -763,10 +756,10 @@ template <class R, int DIR>
 __device__ __forceinline__ void hlle(const R (&leftst)[NVEC], const R (&rigtst)[NVEC], R (&nflux)[NCONS]) {
   const R csl = leftst[mcsp], csr = rigtst[mcsp];
   const R vl = leftst[mvel], vr = rigtst[mvel];
-  R sl = smin(vl, vr) - smax(csl, csr);
-  sl = smin(R(0), sl);
-  R sr = smax(vl, vr) + smax(csl, csr);
-  sr = smax(R(0), sr);
+  R sl = xmin(vl, vr) - xmax(csl, csr);
+  sl = xmin(R(0), sl);
+  R sr = xmax(vl, vr) + xmax(csl, csr);
+  sr = xmax(R(0), sr);
   if constexpr (kFast) {
     const R inv = fdiv(R(1), sr - sl);
 #pragma unroll
@@ -775,7 +768,7 @@ __device__ __forceinline__ void hlle(const R (&leftst)[NVEC], const R (&rigtst)[
   } else {
 #pragma unroll
     for (int m = 0; m < NCONS; m++)
-      nflux[m] = (sr * leftst[NCONS + m] - sl * rigtst[NCONS + m] + sl * sr * (rigtst[m] - leftst[m])) / (sr - sl);
+      nflux[m] = fdiv(sr * leftst[NCONS + m] - sl * rigtst[NCONS + m] + sl * sr * (rigtst[m] - leftst[m]), sr - sl);
   }
 }
 
@@ -796,15 +789,15 @@ __device__ __forceinline__ void hllc(const R (&leftst)[NVEC], const R (&rigtst)[
     vxl = Pl[D::nved]; vyl = Pl[D::nvef]; vzl = Pl[D::nveb];
     vxr = Pr[D::nved]; vyr = Pr[D::nvef]; vzr = Pr[D::nveb];
   } else {
-    vxl = leftst[muvu] / leftst[mudn]; vyl = leftst[muvv] / leftst[mudn]; vzl = leftst[muvw] / leftst[mudn];
-    vxr = rigtst[muvu] / rigtst[mudn]; vyr = rigtst[muvv] / rigtst[mudn]; vzr = rigtst[muvw] / rigtst[mudn];
+    vxl = fdiv(leftst[muvu], rol); vyl = fdiv(leftst[muvv], rol); vzl = fdiv(leftst[muvw], rol);
+    vxr = fdiv(rigtst[muvu], ror); vyr = fdiv(rigtst[muvv], ror); vzr = fdiv(rigtst[muvw], ror);
   }
   const R scl = leftst[must], scr = rigtst[must];
   const R byl = leftst[mubv], bzl = leftst[mubw], byr = rigtst[mubv], bzr = rigtst[mubw];
   const R ptl = leftst[mpre], ptr = rigtst[mpre];
   const R cfl = leftst[mcsp], cfr = rigtst[mcsp];
-  const R sl = smin(vxl, vxr) - smax(cfl, cfr);
-  const R sr = smax(vxl, vxr) + smax(cfl, cfr);
+  const R sl = xmin(vxl, vxr) - xmax(cfl, cfr);
+  const R sr = xmax(vxl, vxr) + xmax(cfl, cfr);
   const R sdl = sl - vxl, sdr = sr - vxr;
   const R rosdl = rol * sdl, rosdr = ror * sdr;
   const R temp = fdiv(R(1), rosdr - rosdl);
@@ -822,8 +815,8 @@ __device__ __forceinline__ void hllc(const R (&leftst)[NVEC], const R (&rigtst)[
   const R byrst = rorst / ror * byr, bzrst = rorst / ror * bzr, scrst = rorst / ror * scr;
   const R eerst = (sdr * eer - ptr * vxr + ptst * sm) * isdmr;
   const R sign1 = copysign(R(1), sm);
-  const R maxs1 = smax(R(0), sign1), mins1 = -smin(R(0), sign1);
-  const R msl = smin(sl, R(0)), msr = smax(sr, R(0));
+  const R maxs1 = xmax(R(0), sign1), mins1 = -xmin(R(0), sign1);
+  const R msl = xmin(sl, R(0)), msr = xmax(sr, R(0));
   nflux[mden] = (leftst[mfdn] + msl * (rolst - rol)) * maxs1 + (rigtst[mfdn] + msr * (rorst - ror)) * mins1;
   nflux[meto] = (leftst[mfet] + msl * (eelst - eel)) * maxs1 + (rigtst[mfet] + msr * (eerst - eer)) * mins1;
   nflux[mrvu] = (leftst[mfvu] + msl * (rxlst - rxl)) * maxs1 + (rigtst[mfvu] + msr * (rxrst - rxr)) * mins1;
@@ -879,7 +872,7 @@ __device__ __forceinline__ void face_flux(const R (&Pl)[NPRIM], const R (&Pr)[NP
       return;
     }
   }
-  if (branch_hlld && riemann == RIEMANN_HLLD) {  // the upwind flux is formed inside hlld_branch
+  if (riemann == RIEMANN_HLLD) {  // the upwind flux is formed inside hlld_branch / hlld
     prim2cons_state<R, DIR>(Pl, Cl, rot);
     prim2cons_state<R, DIR>(Pr, Cr, rot);
   } else {
@@ -892,7 +885,7 @@ __device__ __forceinline__ void face_flux(const R (&Pl)[NPRIM], const R (&Pr)[NP
     hllc<R, DIR>(Cl, Cr, Pl, Pr, nf);
   } else {
     if constexpr (branch_hlld) hlld_branch<R, DIR>(Cl, Cr, Pl, Pr, nf, rot);
-    else hlld<R, DIR>(Cl, Cr, Pl, Pr, nf);
+    else hlld<DIR>(Cl, Cr, Pl, Pr, nf, rot);
   }
   F[mden] = nf[mden];
   F[mrv1] = nf[D::orv1];
@@ -902,21 +895,21 @@ __device__ __forceinline__ void face_flux(const R (&Pl)[NPRIM], const R (&Pr)[NP
   // HLLD output slots for the two tangential fields (numflux[mbmv]/[mbmw] = slots 6/7)
   F[D::ob_a] = nf[D::sb_a];
   F[D::ob_b] = nf[D::sb_b];
-  F[D::glm] = R(0.5) * (Cl[mubp] + Cr[mubp]) - R(0.5) * chg * (Cr[mubu] - Cl[mubu]);
+  F[D::glm] = half_of(Cl[mubp] + Cr[mubp]) - R(0.5) * chg * (Cr[mubu] - Cl[mubu]);
   if constexpr (kFast && std::is_same<R, double>::value) {  // hoisted 0.5/c_h and c_h^2
     F[mbps] = (R(0.5) * (Cl[mubu] + Cr[mubu]) - g.hoc * (Cr[mubp] - Cl[mubp])) * g.chg2;
   } else if constexpr (kFast) {  // FP32: recomputed per face (cheap, and two fewer live registers)
     F[mbps] = (R(0.5) * (Cl[mubu] + Cr[mubu]) - fdiv(R(0.5), chg) * (Cr[mubp] - Cl[mubp])) * chg * chg;
   } else {  // the reference's order: ((...) * chg) * chg
-    F[mbps] = (R(0.5) * (Cl[mubu] + Cr[mubu]) - g.hoc * (Cr[mubp] - Cl[mubp])) * chg * chg;
+    F[mbps] = (half_of(Cl[mubu] + Cr[mubu]) - g.hoc * (Cr[mubp] - Cl[mubp])) * chg * chg;
   }
   F[mst] = nf[mst];
 }
 
 // Left state of face c+1/2 and right state of face c-1/2 from cell value p and limited slope s
 // (mhd.cpp:1139 and 1153).
-template <class R> __device__ __forceinline__ R left_state(R p, R s) { return p + R(0.5) * s; }
-template <class R> __device__ __forceinline__ R right_state(R p, R s) { return p - R(0.5) * s; }
+template <class R> __device__ __forceinline__ R left_state(R p, R s) { return p + half_of(s); }
+template <class R> __device__ __forceinline__ R right_state(R p, R s) { return p - half_of(s); }
 
 // UpdatePrimitvP for one cell, mhd.cpp:1483-1506.  u: 10 conserved values -> p: 12 primitives.
 template <class R>
@@ -932,8 +925,8 @@ __device__ __forceinline__ void cons2prim(const R (&u)[NCONS], R gam, R (&p)[NPR
   if constexpr (kFast) {  // (E - m^2 / (2 rho) - B^2 / 2) / rho in two FMAs
     p[nene] = fma(R(-0.5) * rhoinv, m2, fma(R(-0.5), b2, u[meto])) * rhoinv;
   } else {
-    const R ekin = R(0.5) * m2 * rhoinv, emag = R(0.5) * b2;
-    p[nene] = (u[meto] - ekin - emag) / u[mden];
+    const R ekin = half_of(m2) * rhoinv, emag = half_of(b2);
+    p[nene] = fdiv(u[meto] - ekin - emag, u[mden]);
   }
   p[npre] = p[nene] * p[nden] * (gam - R(1));
   p[ncsp] = fsqrt_est(p[nene] * gam * (gam - R(1)));  // the sound speed only enters wave-speed estimates
@@ -952,9 +945,7 @@ __device__ __forceinline__ R cell_dt(const R (&p)[NPRIM], R dx, R dy, R dz) {
   const R b = fdiv_est(dy, fabs(p[nve2]) + ctot);
   const R c = fdiv_est(dz, fabs(p[nve3]) + ctot);
   if constexpr (kFast && std::is_same<R, double>::value) return imin(imin(dt, b), c);  // integer pipe
-  if (b < dt) dt = b;
-  if (c < dt) dt = c;
-  return dt;
+  return xmin(xmin(dt, b), c);
 }
 
 // Per-cell maximum signal speed (EvaluateCh, mhd.cpp:1589-1601).
@@ -962,21 +953,19 @@ template <class R>
 __device__ __forceinline__ R cell_ch(const R (&p)[NPRIM]) {
   const R css = p[ncsp] * p[ncsp];
   const R ri = kFast ? fdiv_est(R(1), p[nden]) : R(0);  // fast form: one reciprocal of rho
-  const R ca1 = kFast ? p[nbm1] * p[nbm1] * ri : p[nbm1] * p[nbm1] / p[nden];
-  const R ca2 = kFast ? p[nbm2] * p[nbm2] * ri : p[nbm2] * p[nbm2] / p[nden];
-  const R ca3 = kFast ? p[nbm3] * p[nbm3] * ri : p[nbm3] * p[nbm3] / p[nden];
+  const R ca1 = kFast ? p[nbm1] * p[nbm1] * ri : fdiv(p[nbm1] * p[nbm1], p[nden]);
+  const R ca2 = kFast ? p[nbm2] * p[nbm2] * ri : fdiv(p[nbm2] * p[nbm2], p[nden]);
+  const R ca3 = kFast ? p[nbm3] * p[nbm3] * ri : fdiv(p[nbm3] * p[nbm3], p[nden]);
   const R cts = css + ca1 + ca2 + ca3;
-  const R cm1 = fsqrt_est((cts + fsqrt_est(cts * cts - R(4) * css * ca1)) / R(2));
+  const R cm1 = fsqrt_est(half_of(cts + fsqrt_est(cts * cts - R(4) * css * ca1)));
   const R ch1 = (fabs(p[nve1]) + cm1);
-  const R cm2 = fsqrt_est((cts + fsqrt_est(cts * cts - R(4) * css * ca2)) / R(2));
+  const R cm2 = fsqrt_est(half_of(cts + fsqrt_est(cts * cts - R(4) * css * ca2)));
   const R ch2 = (fabs(p[nve2]) + cm2);
-  const R cm3 = fsqrt_est((cts + fsqrt_est(cts * cts - R(4) * css * ca3)) / R(2));
+  const R cm3 = fsqrt_est(half_of(cts + fsqrt_est(cts * cts - R(4) * css * ca3)));
   const R ch3 = (fabs(p[nve3]) + cm3);
   R m = ch1;
   if constexpr (kFast && std::is_same<R, double>::value) return imax(imax(m, ch2), ch3);  // integer pipe
-  if (m < ch2) m = ch2;
-  if (m < ch3) m = ch3;
-  return m;
+  return xmax(xmax(m, ch2), ch3);
 }
 
 }  // namespace MHDGB_VNS

@@ -84,7 +84,7 @@ __global__ void k_damp_psi(double* __restrict__ U, Layout L, const double* __res
   double dhl = dxs[i];
   if (dys[j] < dhl) dhl = dys[j];
   if (dzs[k] < dhl) dhl = dzs[k];
-  const double taui = alphabp * *chg_ptr / dhl;
+  const double taui = fdiv(alphabp * *chg_ptr, dhl);
   const size_t c = L.at(NCONS, mbps, k, j, i);
   U[c] = U[c] * (1.0 - *dt_ptr * taui);
 }
