@@ -229,10 +229,11 @@ MHDGB_HD double van_leer_split(double dp, double dm, bool& ok) {
   const unsigned hp = d_hi(dp), hm = d_hi(dm), ap = hp & 0x7FFFFFFFu, am = hm & 0x7FFFFFFFu;
   const unsigned top = u_max(ap, am);
   constexpr unsigned lo_lim = (1023u - 700u) << 20, hi_lim = 0x7FF00000u;
-  ok = ok && top - lo_lim < hi_lim - lo_lim;
+  const bool zero = (top | d_lo(dp) | d_lo(dm)) == 0u;  // a uniform stretch: common, and exact
+  ok = ok && (zero || top - lo_lim < hi_lim - lo_lim);
   const unsigned base = (top & 0x7FF00000u) - (127u << 20);  // the larger one scaled into [1, 2)
   // opposite signs, or the smaller one below 2^-71 of the larger: no slope
-  const bool flat = (int)(hp ^ hm) < 0 || (int)(u_min(ap, am) - base) < (56 << 20);
+  const bool flat = zero || (int)(hp ^ hm) < 0 || (int)(u_min(ap, am) - base) < (56 << 20);
   auto scaled = [base](unsigned a, unsigned lo) {  // as p_narrow_nz
     const unsigned f = f_shl(a - base, lo, 3);
     return Pair{f_from(f + ((lo >> 28) & 1u)), f_mul(i_to_f((int)(lo << 3)), f_from((f & 0x7F800000u) - (55u << 23)))};
