@@ -38,8 +38,9 @@
 namespace mhdgb {
 
 // Bounds within which the pairs neither overflow nor lose their low parts: density and sound speed
-// in [2^-20, 2^20], velocities and fields below 2^20, tangential fields zero or above 2^-83 (pressure
-// and energy follow from density and sound speed; a NaN in them is one in the sound speed).  Other
+// in [2^-20, 2^20], velocities and fields below 2^20, the larger tangential field component zero or
+// above 2^-83 (pressure and energy follow from density and sound speed; a NaN in them is one in the
+// sound speed).  Other
 // faces (and those where an outer wave nearly meets the contact) take the general FP64 flux.
 constexpr unsigned kSplitMax = (1023u + 20u) << 20, kSplitMin = (1023u - 20u) << 20, kSplitTinyB = (1023u - 83u) << 20;
 
@@ -54,18 +55,18 @@ MHDGB_HD bool face_flux_split(const double (&Pl)[NPRIM], const double (&Pr)[NPRI
                               double chg2, double (&F)[NCONS], bool hllc) {
   bool ok;  // (checked at the end: a branch here would keep the loads and conversions below from overlapping)
   {
-    unsigned mx = 0, mb = 0xFFFFFFFFu;
-    const int q[] = {nve1, nve2, nve3, nbm1, nbm2, nbm3, nden, ncsp};
+    unsigned mb = 0;
 #pragma unroll
-    for (int n = 0; n < 8; n++) mx = u_max(mx, u_max(d_mag(Pl[q[n]]), d_mag(Pr[q[n]])));
+    for (int n = nbm2; n <= nbm3; n++) mb = u_max(mb, u_max(d_mag(Pl[n]), d_mag(Pr[n])));
+    unsigned mx = mb;
+    const int q[] = {nve1, nve2, nve3, nbm1, nden, ncsp};
 #pragma unroll
-    for (int n = nbm2; n <= nbm3; n++)  // minus one: a zero counts as large
-      mb = u_min(mb, u_min(d_mag(Pl[n]) - 1u, d_mag(Pr[n]) - 1u));
+    for (int n = 0; n < 6; n++) mx = u_max(mx, u_max(d_mag(Pl[q[n]]), d_mag(Pr[q[n]])));
     // signed comparison: a negative value fails
     const int mn = (int)kSplitMin;
     const bool pos = (int)d_hi(Pl[nden]) >= mn && (int)d_hi(Pr[nden]) >= mn && (int)d_hi(Pl[ncsp]) >= mn &&
                      (int)d_hi(Pr[ncsp]) >= mn;
-    ok = mx < kSplitMax && mb >= kSplitTinyB && pos;
+    ok = mx < kSplitMax && mb - 1u >= kSplitTinyB - 1u && pos;  // (mb = 0 passes)
   }
   const Pair rl = p_narrow_nz(Pl[nden]), rr = p_narrow_nz(Pr[nden]);
   const Pair bxl = p_narrow(Pl[nbm1]), bxr = p_narrow(Pr[nbm1]);

@@ -1,7 +1,7 @@
 """The FP64 form's face flux in FP32 pairs against the oracle where its dispatch and its range end.
 
 The pairs take faces whose density and sound speed lie in [2^-20, 2^20], with velocities and fields
-below 2^20 and tangential fields zero or above 2^-83; others take the general FP64 flux.  The states
+below 2^20 and the larger tangential field component zero or above 2^-83; others take the general FP64 flux.  The states
 are one smooth state in other units: density times R, velocity times V, field times sqrt(R) V b,
 pressure times R V^2, placed inside the range, outside it, and across its ends (both fluxes side by
 side).  Tolerance: a flux in pairs is within 2^-43 of FP64 relative to its own terms, and a step adds
