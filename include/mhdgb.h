@@ -171,8 +171,9 @@ int mhdgb_reset_clock(mhdgb_solver* h);
  * steps, download the new U and return the step's dt and c_h.  The drop-in form of the loop body
  * for callers that keep the state on the host.  Page-locked, mapped arrays (cudaHostAlloc,
  * cudaHostRegister, a pinned torch tensor) are read and written by the kernels themselves over the
- * host link: the recovery pass reads U_in, the last step writes each updated cell of U_out, and the
- * ghost cells of a separate U_out are copied from U_in.  Other arrays go through a device staging
+ * host link (FP64 forms: the recovery pass reads U_in and the last step writes each updated cell of
+ * U_out; mixed form: repacking passes before and after), and the ghost cells of a separate U_out are
+ * U_in's.  Other arrays go through a device staging
  * buffer.  Both give the same U_out bit for bit; U_out may be U_in. */
 int mhdgb_step_host(mhdgb_solver* h, const double* U_in, double* U_out, int nsteps, double* dt, double* chg);
 

@@ -737,7 +737,7 @@ k_fused_step(const InstanceDesc* __restrict__ desc, LaunchCtrl* __restrict__ lc)
         update_cell(acc, a.U + c0, fsU, dt, chd, dtf, chf, a, ii + NGH, jj + NGH, k + NGH, u);
 #pragma unroll
         for (int m = 0; m < NCONS; m++) a.U[c0 + m * fsU] = u[m];
-        if (a.Uh) {  // the caller's host copy of U (end-to-end steps), field stride itot
+        if (sizeof(R) == sizeof(double) && a.Uh) {  // the caller's host copy of U (FP64 end-to-end steps), field stride itot
           double* uh = a.Uh + ((size_t)(ii + NGH) + (size_t)L.itot * NCONS * ((size_t)(jj + NGH) +
                                                                             (size_t)L.jtot * (size_t)(k + NGH)));
 #pragma unroll

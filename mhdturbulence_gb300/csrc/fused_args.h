@@ -35,7 +35,7 @@ struct FusedArgs {
   // takes all tiles of chunk 0 first, so chunks that shrink with c even out the CTAs' finish times
   int kst[MAX_ZCHUNKS + 1];
   Ctrl* ctrl;
-  // End-to-end steps: the caller's host array of U (reference layout, itot x jtot x ktot, reached
+  // End-to-end steps of the FP64 forms: the caller's host array of U (reference layout, itot x jtot x ktot, reached
   // over the host link), written by the step's cell updates besides U; null otherwise.
   double* Uh;
   // Bytes the first plane load of each work item is expected to deliver beyond the plane itself:

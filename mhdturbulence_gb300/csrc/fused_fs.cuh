@@ -275,12 +275,6 @@ k_fused_step_fs(const InstanceDesc* __restrict__ desc, LaunchCtrl* __restrict__ 
         update_cell(acc, a.U + cu, fsU, dt, chd, dtf, chf, a, ii + NGH, jj + NGH, k + NGH, u);
 #pragma unroll
         for (int m = 0; m < NCONS; m++) a.U[cu + m * fsU] = u[m];
-        if (a.Uh) {  // the caller's host copy of U (end-to-end steps), field stride itot
-          double* uh = a.Uh + ((size_t)(ii + NGH) + (size_t)L.itot * NCONS * ((size_t)(jj + NGH) +
-                                                                            (size_t)L.jtot * (size_t)(k + NGH)));
-#pragma unroll
-          for (int m = 0; m < NCONS; m++) uh[(size_t)m * L.itot] = u[m];
-        }
         R dtc, chc;
         recover_cell<R>(u, a.gam, Pout, L, a.bc, ii, jj, k, spacing_of<R>(a, 0, ii + NGH),
                         spacing_of<R>(a, 1, jj + NGH), spacing_of<R>(a, 2, k + NGH), dtc, chc, bad);
