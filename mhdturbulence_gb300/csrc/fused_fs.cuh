@@ -265,10 +265,14 @@ k_fused_step_fs(const InstanceDesc* __restrict__ desc, LaunchCtrl* __restrict__ 
         const R yi = inv_of<R>(a, 1, (a.quirk ? ii : jj) + NGH);
         const R zi = inv_of<R>(a, 2, (a.quirk ? ii : k) + NGH);
 #pragma unroll
-        for (int m = 0; m < NCONS; m++) {
-          acc.first(m, FXS(fb, m, oi + 1, oj) - FXS(fb, m, oi, oj), xi);
-          acc.add(m, FYS(fb, m, oi, oj + 1) - FYS(fb, m, oi, oj), yi);
-          acc.add(m, FZS(zh, m, oi, oj) - FZS(zl, m, oi, oj), zi);
+        for (int q = 0; q < NCONS / 2; q++) {
+          const int m = 2 * q;
+          acc.first(q, make_float2(FXS(fb, m, oi + 1, oj), FXS(fb, m + 1, oi + 1, oj)),
+                    make_float2(FXS(fb, m, oi, oj), FXS(fb, m + 1, oi, oj)), xi);
+          acc.add(q, make_float2(FYS(fb, m, oi, oj + 1), FYS(fb, m + 1, oi, oj + 1)),
+                  make_float2(FYS(fb, m, oi, oj), FYS(fb, m + 1, oi, oj)), yi);
+          acc.add(q, make_float2(FZS(zh, m, oi, oj), FZS(zh, m + 1, oi, oj)),
+                  make_float2(FZS(zl, m, oi, oj), FZS(zl, m + 1, oi, oj)), zi);
         }
         const size_t cu = L.at(NCONS, 0, k + NGH, jj + NGH, ii + NGH);
         double u[NCONS];
