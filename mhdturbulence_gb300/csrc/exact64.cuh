@@ -7,7 +7,8 @@
 // 53-bit numbers is never a tie.  About 70 integer and FP32 instructions against eight to ten FP64
 // instructions, each of which keeps a sub-partition's FP64 path busy for 65 cycles.  With halvings,
 // comparisons and HLLD's masks off the FP64 pipe too, the three flux kernels of a 64x96x48 stage step
-// went from 1.47 to 0.78 ms and a fused step of 100x62x90 from 4.75 to 3.4 ms, bit for bit the same.
+// went from 1.47 to 0.71 ms and a fused step of 100x62x90 from 4.75 to 2.99 ms, bit for bit the same (0.78
+// and 3.40 with a branch in every division).
 #pragma once
 
 #include "fp32pair.cuh"
@@ -25,12 +26,14 @@ MHDGB_HD Pair significand_pair(unsigned hi, unsigned lo) {
   return Pair{f_from((f_shl(hi, lo, 3) & 0x007FFFFFu) | 0x3F800000u), f_mul(i_to_f((int)(lo & 0x1FFFFFFFu)), 0x1p-52f)};
 }
 
-// a / b, rounded to nearest even.  Zeros, subnormal, infinite and NaN operands and results near the ends
-// of the exponent range take the division instruction sequence.
-MHDGB_HD double div_rn(double a, double b) {
+// a / b, rounded to nearest even, without a branch; ok becomes false for subnormal, infinite and NaN
+// operands, zero divisors and results near the ends of the exponent range (the result is then
+// meaningless).  Several of these overlap where a branch in each would run them one after the other.
+MHDGB_HD double div_core(double a, double b, bool& ok) {
   const unsigned ha = d_hi(a), la = d_lo(a), hb = d_hi(b), lb = d_lo(b);
   const int ea = (int)((ha >> 20) & 0x7FFu), eb = (int)((hb >> 20) & 0x7FFu), er = ea - eb + 1023;
-  if ((unsigned)(ea - 1) >= 2046u || (unsigned)(eb - 1) >= 2046u || (unsigned)(er - 2) >= 2044u) return a / b;
+  const bool zero = ((ha << 1) | la) == 0u;
+  ok = ok && (unsigned)(eb - 1) < 2046u && (zero || ((unsigned)(ea - 1) < 2046u && (unsigned)(er - 2) < 2044u));
   const unsigned long long B = ((unsigned long long)((hb & 0xFFFFFu) | 0x100000u) << 32) | lb;
   const unsigned ma = ha & 0xFFFFFu, mb = hb & 0xFFFFFu;
   const bool s = ma < mb || (ma == mb && la < lb);  // significand quotient below 1: scale a by 2
@@ -48,13 +51,15 @@ MHDGB_HD double div_rn(double a, double b) {
   Q += (2 * R > (long long)B ? 1 : 0) - (2 * R < -(long long)B ? 1 : 0);
   const unsigned long long bits =
       (unsigned long long)Q + ((unsigned long long)(unsigned)(er - 1 - (s ? 1 : 0)) << 52);
-  return d_from((unsigned)(bits >> 32) | ((ha ^ hb) & 0x80000000u), (unsigned)bits);
+  const unsigned sign = (ha ^ hb) & 0x80000000u;
+  return d_from(zero ? sign : (unsigned)(bits >> 32) | sign, zero ? 0u : (unsigned)bits);
 }
 
-// sqrt(x), rounded to nearest even; zero, subnormal, negative, infinite and NaN arguments as div_rn.
-MHDGB_HD double sqrt_rn(double x) {
+// sqrt(x), rounded to nearest even, as div_core; zero, subnormal, negative, infinite and NaN arguments are
+// left to the caller.
+MHDGB_HD double sqrt_core(double x, bool& ok) {
   const unsigned hx = d_hi(x), lx = d_lo(x);
-  if (hx - 0x00100000u >= 0x7FE00000u) return sqrt(x);
+  ok = ok && hx - 0x00100000u < 0x7FE00000u;
   const int e = (int)(hx >> 20) - 1023, p = e & 1;
   const Pair m = significand_pair(hx, lx);
   const float two = p ? 2.0f : 1.0f;
@@ -68,6 +73,37 @@ MHDGB_HD double sqrt_rn(double x) {
   Q += (R > Q ? 1 : 0) - (R <= -Q ? 1 : 0);
   const unsigned long long bits = (unsigned long long)Q + ((unsigned long long)(unsigned)((e - p) / 2 + 1022) << 52);
   return d_from((unsigned)(bits >> 32), (unsigned)bits);
+}
+
+// The instruction sequences, out of line, for what the cores leave.
+inline __host__ __device__ __noinline__ double div_ieee(double a, double b) { return a / b; }
+inline __host__ __device__ __noinline__ double sqrt_ieee(double x) { return sqrt(x); }
+
+MHDGB_HD double div_rn(double a, double b) {
+  bool ok = true;
+  const double q = div_core(a, b, ok);
+  return ok ? q : div_ieee(a, b);
+}
+MHDGB_HD double sqrt_rn(double x) {
+  bool ok = true;
+  const double q = sqrt_core(x, ok);
+  return ok ? q : sqrt_ieee(x);
+}
+// N divisions with one test for all.
+template <int N>
+MHDGB_HD void div_many(const double (&a)[N], const double (&b)[N], double (&q)[N]) {
+  unsigned left = 0;
+#pragma unroll
+  for (int i = 0; i < N; i++) {
+    bool ok = true;
+    q[i] = div_core(a[i], b[i], ok);
+    left |= ok ? 0u : 1u << i;
+  }
+  if (left) {
+#pragma unroll
+    for (int i = 0; i < N; i++)
+      if ((left >> i) & 1u) q[i] = div_ieee(a[i], b[i]);
+  }
 }
 
 }  // namespace mhdgb

@@ -242,6 +242,11 @@ __device__ __forceinline__ double twice_div_est(double p, double s) {
 // van_leer(P[c+1]-P[c], P[c]-P[c-1]); the reference evaluates the same expression for the left
 // state of face c+1/2 and the right state of face c-1/2 (mhd.cpp:1134-1154), so one evaluation
 // per cell and direction gives both.
+// 2 a b rounded as (2 a) b, from p = a b > 0: twice p unless p is subnormal or twice it overflows.
+__device__ __forceinline__ double twice_product(double p, double a, double b) {
+  const unsigned e = (unsigned)__double2hiint(p) >> 20;
+  return e - 1u < 2045u ? d_from(d_hi(p) + (1u << 20), d_lo(p)) : 2.0 * a * b;
+}
 // van_leer_general: the FP64 fast build's expression for the arguments van_leer_split leaves, out of line.
 __device__ __noinline__ double van_leer_general(double dsvp, double dsvm) {
   const double p = dsvp * dsvm;
@@ -260,9 +265,7 @@ __device__ __forceinline__ R van_leer(R dsvp, R dsvm) {
     }
   } else {
     const R p = dsvp * dsvm;
-    if (!pos_nonzero(p)) return R(0);
-    const unsigned e = (unsigned)__double2hiint(p) >> 20;  // 2 dsvp dsvm is 2 p unless p is subnormal
-    return fdiv(e - 1u < 2045u ? d_from(d_hi(p) + (1u << 20), d_lo(p)) : R(2) * dsvp * dsvm, dsvp + dsvm);
+    return pos_nonzero(p) ? fdiv(twice_product(p, dsvp, dsvm), dsvp + dsvm) : R(0);
   }
 }
 
@@ -283,6 +286,21 @@ __device__ __forceinline__ void van_leer_batch(const R (&dp)[N], const R (&dm)[N
       for (int n = 0; n < N; n++)
         if ((left >> n) & 1u) s[n] = van_leer_general(dp[n], dm[n]);
     }
+  } else if constexpr (std::is_same<R, double>::value) {  // the exact build: van_leer's steps, one test for all
+    double num[N], den[N];
+    bool on[N];
+#pragma unroll
+    for (int n = 0; n < N; n++) {
+      const double p = dp[n] * dm[n];
+      on[n] = pos_nonzero(p);
+      num[n] = twice_product(p, dp[n], dm[n]);
+      den[n] = dp[n] + dm[n];
+      if (!on[n]) {  // 0 / 1
+        num[n] = 0.0;
+        den[n] = 1.0;
+      }
+    }
+    div_many<N>(num, den, s);
   } else {
 #pragma unroll
     for (int n = 0; n < N; n++) s[n] = van_leer<R>(dp[n], dm[n]);
@@ -494,10 +512,13 @@ __device__ __forceinline__ void hlld(const double (&leftst)[NVEC], const double 
                                      int rot = 0) {
   using R = double;
   const R eps = 1.0e-30;
-  const R vxl = fdiv(leftst[muvu], leftst[mudn]), vyl = fdiv(leftst[muvv], leftst[mudn]),
-          vzl = fdiv(leftst[muvw], leftst[mudn]);
-  const R vxr = fdiv(rigtst[muvu], rigtst[mudn]), vyr = fdiv(rigtst[muvv], rigtst[mudn]),
-          vzr = fdiv(rigtst[muvw], rigtst[mudn]);
+  R v6[6];
+  {
+    const R num[6] = {leftst[muvu], leftst[muvv], leftst[muvw], rigtst[muvu], rigtst[muvv], rigtst[muvw]};
+    const R den[6] = {leftst[mudn], leftst[mudn], leftst[mudn], rigtst[mudn], rigtst[mudn], rigtst[mudn]};
+    div_many<6>(num, den, v6);
+  }
+  const R vxl = v6[0], vyl = v6[1], vzl = v6[2], vxr = v6[3], vyr = v6[4], vzr = v6[5];
   const R ptl = leftst[mpre], ptr = rigtst[mpre];
   // Step 1 (mhd.cpp:212-216)
   const R cfast = xmax(leftst[mcsp], rigtst[mcsp]);
@@ -518,12 +539,10 @@ __device__ __forceinline__ void hlld(const double (&leftst)[NVEC], const double 
     R ro, vx, vy, vz, by, bz, isdm;
     bool nondeg;
   };
-  auto star = [&](R ro, R vx, R vy, R vz, R by, R bz, R sd, R rosd, R sdm) {
+  auto star = [&](R ro, R vx, R vy, R vz, R by, R bz, R sd, R rosd, R sdm, R f, R isdm, R itf) {
     Star t;
-    t.isdm = fdiv(1.0, sdm);
-    const R f = rosd * sdm - bxsq;
+    t.isdm = isdm;
     t.nondeg = !abs_less(f, eps);
-    const R itf = fdiv(1.0, f);
     const R t1 = bxs * (sd - sdm) * itf, t2 = (rosd * sd - bxsq) * itf;
     t.ro = t.nondeg ? rosd * t.isdm : ro;
     t.vx = t.nondeg ? sm : vx;
@@ -541,10 +560,18 @@ __device__ __forceinline__ void hlld(const double (&leftst)[NVEC], const double 
   for (int n = 0; n < NPRIM; n++) pup[n] = sel(Pl[n], Pr[n]);
   const R ro = cst[mudn], by = cst[mubv], bz = cst[mubw], ee = cst[muet], pt = cst[mpre];
   const R vx = sel(vxl, vxr), vy = sel(vyl, vyr), vz = sel(vzl, vzr), sd = sel(sdl, sdr);
-  const Star u = star(ro, vx, vy, vz, by, bz, sd, sel(rosdl, rosdr), sel(sdml, sdmr));
+  const R fl = rosdl * sdml - bxsq, fr = rosdr * sdmr - bxsq;
+  R inv4[4];  // a degenerate side's 1 / f is not used
+  {
+    const R one[4] = {1.0, 1.0, 1.0, 1.0};
+    const R den[4] = {sdml, sdmr, abs_less(fl, eps) ? 1.0 : fl, abs_less(fr, eps) ? 1.0 : fr};
+    div_many<4>(one, den, inv4);
+  }
+  const Star u = star(ro, vx, vy, vz, by, bz, sd, sel(rosdl, rosdr), sel(sdml, sdmr), sel(fl, fr),
+                      sel(inv4[0], inv4[1]), sel(inv4[2], inv4[3]));
   const Star o = star(sel(rigtst[mudn], leftst[mudn]), sel(vxr, vxl), sel(vyr, vyl), sel(vzr, vzl),
                       sel(rigtst[mubv], leftst[mubv]), sel(rigtst[mubw], leftst[mubw]), sel(sdr, sdl),
-                      sel(rosdr, rosdl), sel(sdmr, sdml));
+                      sel(rosdr, rosdl), sel(sdmr, sdml), sel(fr, fl), sel(inv4[1], inv4[0]), sel(inv4[3], inv4[2]));
   const R rost = u.ro, rxst = rost * u.vx, ryst = rost * u.vy, rzst = rost * u.vz;
   const R vdbst = u.vx * bxs + u.vy * u.by + u.vz * u.bz;
   R eest = ee;
@@ -555,12 +582,22 @@ __device__ __forceinline__ void hlld(const double (&leftst)[NVEC], const double 
   // Step 5C (mhd.cpp:338-377) and the Alfven speed of Step 6 (mhd.cpp:381-383)
   R rydst = ryst, rzdst = rzst, bydst = u.by, bzdst = u.bz, eedst = eest, sst = 0.0;
   if (!abs_less(bxs, eps)) {
-    const R sq = fsqrt(rost), sqo = fsqrt(o.ro);
+    bool ok = true;
+    R sq = sqrt_core(rost, ok), sqo = sqrt_core(o.ro, ok);
+    if (!ok) {
+      sq = sqrt_ieee(rost);
+      sqo = sqrt_ieee(o.ro);
+    }
     const R ql = sel(sq, sqo), qr = sel(sqo, sq);
     const R vylst = sel(u.vy, o.vy), vyrst = sel(o.vy, u.vy), vzlst = sel(u.vz, o.vz), vzrst = sel(o.vz, u.vz);
     const R bylst = sel(u.by, o.by), byrst = sel(o.by, u.by), bzlst = sel(u.bz, o.bz), bzrst = sel(o.bz, u.bz);
     const bool neg = signbit(bxs);
-    const R inv = fdiv(1.0, ql + qr);
+    R is[2];
+    {
+      const R num[2] = {1.0, fabs(bxs)}, den[2] = {ql + qr, sq};
+      div_many<2>(num, den, is);
+    }
+    const R inv = is[0];
     const R vydst = inv * (ql * vylst + qr * vyrst + negate_if(byrst - bylst, neg));
     const R vzdst = inv * (ql * vzlst + qr * vzrst + negate_if(bzrst - bzlst, neg));
     const R sqq = negate_if(ql, neg) * qr;
@@ -571,8 +608,7 @@ __device__ __forceinline__ void hlld(const double (&leftst)[NVEC], const double 
     const R vdb = sm * bxs + vydst * bydst + vzdst * bzdst;
     const R de = negate_if(sq, neg) * (vdbst - vdb);
     eedst = left ? eest - de : eest + de;
-    const R sa = fdiv(fabs(bxs), sq);
-    sst = left ? sm - sa : sm + sa;
+    sst = left ? sm - is[1] : sm + is[1];
   }
   // Step 6 (mhd.cpp:384-415)
   const R ms = left ? xmin(sl, 0.0) : xmax(sr, 0.0), msst = left ? xmin(sst, 0.0) : xmax(sst, 0.0);
