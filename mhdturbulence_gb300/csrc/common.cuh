@@ -228,6 +228,17 @@ struct FastDiv {
 __device__ __forceinline__ void prefetch_l2(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
+// Pulls rows of cx <= TX doubles, ip apart from u0 (the fields of a tile's plane: adjacent rows for one j), into
+// L2, one cache line per thread and turn (threads q, q + nt, ... of the block).  A row fills TX / 16 lines and
+// may straddle one more.
+template <int TX>
+__device__ __forceinline__ void prefetch_rows(const double* u0, int ip, int rows, int cx, int q, int nt) {
+  constexpr int NP = TX / 16 + 1;
+  for (; q < rows * NP; q += nt) {
+    const int r = q / NP;
+    prefetch_l2(u0 + (size_t)ip * r + min(16 * (q - r * NP), cx - 1));
+  }
+}
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)map) : "memory");
 }
