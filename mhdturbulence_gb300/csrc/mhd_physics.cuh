@@ -377,7 +377,7 @@ __device__ __forceinline__ R sum_sq3(const R (&P)[NPRIM], int b, int rot) {
 
 // Prim2ConsD, mhd.cpp:997-1076 (note the energy flux term bsq*B_d of mhd.cpp:1049-1050).
 template <class R, int DIR>
-__device__ __forceinline__ void prim2cons(const R (&Prim)[NPRIM], R (&Cons)[NVEC], int rot = 0) {
+__device__ __forceinline__ void prim2cons(const R (&Prim)[NPRIM], R (&Cons)[NVEC], bool left, int rot = 0) {
   using D = Dir<DIR>;
   const R rho = Prim[nden];
   const R rhoinv = fdiv_est(R(1), rho);  // only in the fast-speed estimate below
@@ -402,7 +402,14 @@ __device__ __forceinline__ void prim2cons(const R (&Prim)[NPRIM], R (&Cons)[NVEC
   Cons[mfvu] += ptl;
   Cons[mfbu] = R(0);
   Cons[mfbv] = Prim[D::nbmf] * Prim[D::nved] - Prim[D::nvef] * Prim[D::nbmd];
-  Cons[mfbw] = Prim[D::nbmb] * Prim[D::nved] - Prim[D::nveb] * Prim[D::nbmd];
+  if constexpr (kFast && std::is_same<R, float>::value) {
+    // Which product is rounded before the other is fused in: left to the compiler, it changed with code far
+    // from here, and the mixed form's HLLE and HLLC results with it.
+    const R a = Prim[D::nbmb], b = Prim[D::nved], c = Prim[D::nveb], d = Prim[D::nbmd];
+    Cons[mfbw] = left ? __fmaf_rn(a, b, -__fmul_rn(c, d)) : __fmaf_rn(-c, d, __fmul_rn(a, b));
+  } else {
+    Cons[mfbw] = Prim[D::nbmb] * Prim[D::nved] - Prim[D::nveb] * Prim[D::nbmd];
+  }
   Cons[mfbp] = R(0);
   Cons[mfst] = rho * Prim[nst] * Prim[D::nved];
   const R css = Prim[ncsp] * Prim[ncsp];
@@ -912,8 +919,8 @@ __device__ __forceinline__ void face_flux(const R (&Pl)[NPRIM], const R (&Pr)[NP
     prim2cons_state<R, DIR>(Pl, Cl, rot);
     prim2cons_state<R, DIR>(Pr, Cr, rot);
   } else {
-    prim2cons<R, DIR>(Pl, Cl, rot);
-    prim2cons<R, DIR>(Pr, Cr, rot);
+    prim2cons<R, DIR>(Pl, Cl, true, rot);
+    prim2cons<R, DIR>(Pr, Cr, false, rot);
   }
   if (riemann == RIEMANN_HLLE) {
     hlle<R, DIR>(Cl, Cr, nf);
