@@ -592,23 +592,31 @@ int launch_one(mhdgb_solver* h) {
   return MHDGB_OK;
 }
 
-// Relative cost of one plane of a cx x cy tile: its face and slope work against a full tile's, plus
-// a fixed part (barriers, loads).  Only the ratios matter.
-double tile_plane_cost(int cx, int cy, int tx, int ty) {
+// Relative cost of one plane of a cx x cy tile: its face and slope work against a full tile's, plus a fixed
+// part.  Only the ratios matter.  In a kernel with warps beyond its tile's columns (spare) a plane is a chain
+// of face rounds, cell updates and barriers whose latency a thin tile pays in full: half of the time is
+// fixed.  Where every warp owns cells the work itself dominates.  (With a tenth for all, plans counted on
+// thin tiles that were not there: over 40 grids of 20 000 to 17 M cells the step is 5 % (mixed) and 2 %
+// (FP64) faster with the half, at most 26 % (97x61x75 mixed 122 -> 92 us) and at worst 4 % slower; 150^3
+// and 256^3 are planned as before.  The exact form's 32x4/128 kernel on 100x62x90: 3.19 ms with the
+// tenth, 3.59 with the half.)
+double tile_plane_cost(int cx, int cy, int tx, int ty, bool spare) {
   auto warps = [](int n) { return (double)((n + 31) / 32); };
   const double f = (double)(cy * (cx + 1) + (cy + 1) * cx + cy * cx), ff = (double)(ty * (tx + 1) + (ty + 1) * tx + ty * tx);
   const double sl = warps(cy * (cx + 2)) + warps((cy + 2) * cx) + warps(cy * cx);
   const double sf = warps(ty * (tx + 2)) + warps((ty + 2) * tx) + warps(ty * tx);
-  return 0.1 + 0.9 * (0.75 * f / ff + 0.25 * sl / sf);
+  const double fixed = spare ? 0.5 : 0.1;
+  return fixed + (1.0 - fixed) * (0.75 * f / ff + 0.25 * sl / sf);
 }
+
+bool has_spare_warps(const FusedShape& s) { return s.threads > s.tx * s.ty; }
 
 // Finish time of the slowest of `grid` CTAs that take the work items in queue order (chunk-major,
 // then tile rows, then tiles), each CTA the next item when it finishes its last.  A chunk's start
-// costs about kOverheadPlanes planes more (prologue loads, the extra z faces of its first plane);
-// 1.2 fits the measured times of KH ensembles with 8- to 64-plane items and of eleven chunkings of
-// a 150^3 grid in both forms.
+// costs about kOverheadPlanes planes more (prologue loads, the extra z faces of its first plane):
+// with 1.0 the simulated finish is within 5 % of the measured step on 21 grids from 16^3 to 150^3.
 double simulate_queue(const std::vector<double>& tile_cost, const std::vector<int>& chunks, int grid) {
-  constexpr double kOverheadPlanes = 1.2;
+  constexpr double kOverheadPlanes = 1.0;
   std::vector<double> heap(grid, 0.0);  // min-heap of CTA finish times
   auto cmp = [](double a, double b) { return a > b; };
   for (int c : chunks)
@@ -624,11 +632,11 @@ double simulate_queue(const std::vector<double>& tile_cost, const std::vector<in
 // whose sizes shrink (each chunk about remaining * tiles / (K * grid) planes, or a few chunks each
 // a factor r shorter than the one before, so the queue ends on small items that fill the CTAs'
 // last gaps), the one with the earliest simulated finish.
-std::vector<int> choose_chunks(const Layout& L, int tx, int ty, int ntx, int nty, int grid) {
+std::vector<int> choose_chunks(const Layout& L, int tx, int ty, int ntx, int nty, int grid, bool spare) {
   std::vector<double> cost;
   for (int by = 0; by < nty; by++)
     for (int bx = 0; bx < ntx; bx++)
-      cost.push_back(tile_plane_cost(std::min(tx, L.nx - bx * tx), std::min(ty, L.ny - by * ty), tx, ty));
+      cost.push_back(tile_plane_cost(std::min(tx, L.nx - bx * tx), std::min(ty, L.ny - by * ty), tx, ty, spare));
   const int tiles = ntx * nty, nz = L.nz;
   std::vector<std::vector<int>> cand;
   for (int n = 1; n <= std::min(nz, 32); n++) {
@@ -694,7 +702,7 @@ int use_variant(mhdgb_solver* h, int idx, int kc_fixed = 0) {
     const int kc = (L.nz + nc - 1) / nc;
     for (int k = 0; k < L.nz; k += kc) chunks.push_back(std::min(kc, L.nz - k));
   } else {
-    chunks = choose_chunks(L, h->shape.tx, h->shape.ty, h->ntx, h->nty, h->grid);
+    chunks = choose_chunks(L, h->shape.tx, h->shape.ty, h->ntx, h->nty, h->grid, has_spare_warps(h->shape));
   }
   h->nkc = (int)chunks.size();
   h->kst.assign(1, 0);
@@ -1452,7 +1460,7 @@ int mhdgb_plan_zchunks(int nx, int ny, int nz, int tx, int ty, int ctas, int* ch
   L.nx = nx;
   L.ny = ny;
   L.nz = nz;
-  const std::vector<int> c = choose_chunks(L, tx, ty, (nx + tx - 1) / tx, (ny + ty - 1) / ty, ctas);
+  const std::vector<int> c = choose_chunks(L, tx, ty, (nx + tx - 1) / tx, (ny + ty - 1) / ty, ctas, true);
   if ((int)c.size() > max_chunks) return MHDGB_ERR_ARG;
   for (size_t i = 0; i < c.size(); i++) chunks[i] = c[i];
   return (int)c.size();
