@@ -65,8 +65,10 @@ int variants_fp64(const FusedVariant** out) {
       v_fast64::FusedLauncher<double, 32, 4, 128>::variant(FUSED_FP64),
       v_fast64::FusedLauncher<double, 28, 4, 128>::variant(FUSED_FP64),
       v_fast64::FusedLauncher<double, 16, 8, 128>::variant(FUSED_FP64),
-      v_fast64::FusedLauncher<double, 32, 4, 256>::variant(FUSED_FP64),
-      preferred_variant(v_fast64::FusedLauncher<double, 16, 8, 256>::variant(FUSED_FP64)),
+      starting_variant(v_fast64::FusedLauncher<double, 32, 4, 256>::variant(FUSED_FP64), 21.3),
+      starting_variant(preferred_variant(v_fast64::FusedLauncher<double, 16, 8, 256>::variant(FUSED_FP64)), 20.1),
+      // for grids of a few planes per SM: 24x40x20 68 -> 48 us a step, 16^3 44 -> 34 (64^3 322 -> 402)
+      starting_variant(v_fast64::FusedLauncher<double, 8, 8, 256>::variant(FUSED_FP64), 13.2),
       // the run-time solver kernel (HLLE / HLLC); not one of the tuned variants
       v_fast64::FusedLauncher<double, 16, 8, 256, 1, true>::variant(FUSED_FP64),
   };

@@ -70,11 +70,17 @@ struct FusedVariant {
   cudaError_t (*launch)(const InstanceDesc* desc, LaunchCtrl* lc, int grid, cudaStream_t s);
   const char* name;            // kernel form and tile shape, e.g. "two-phase 16x8/256"
   int preferred;               // 1: the entry a grid starts on before any autotuning
+  double plane_us;             // > 0: a smaller grid may start on this entry too; measured time of a full tile's plane
 };
 
 // Marks the table entry a grid starts on: the fastest measured on GB300 at the benchmark sizes.
 inline FusedVariant preferred_variant(FusedVariant v) {
   v.preferred = 1;
+  return v;
+}
+// Marks an entry that grids below the benchmark sizes may start on (the preferred one included).
+inline FusedVariant starting_variant(FusedVariant v, double plane_us) {
+  v.plane_us = plane_us;
   return v;
 }
 

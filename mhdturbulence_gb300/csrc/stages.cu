@@ -348,9 +348,14 @@ cudaError_t launch_ghost_fill(double* P, const Layout& L, const int bc[6], doubl
 namespace detail {
 int variants_exact(const FusedVariant** out) {
   static const FusedVariant v[] = {
-      preferred_variant(v_exact::FusedLauncher<double, 32, 4, 128>::variant(FUSED_FP64_EXACT)),
+      starting_variant(preferred_variant(v_exact::FusedLauncher<double, 32, 4, 128>::variant(FUSED_FP64_EXACT)), 89.3),
+      // One warp on a sub-partition waits for each of its FP64 instructions; with two, the integer arithmetic of
+      // one fills the other's waits: 100x62x90 3.19 -> 2.22 ms a step, 64x96x48 1.60 -> 1.11 (150^3 17.3 ->
+      // 12.1), and with the small tile 24x40x20 192 -> 119 us (100x62x90 2.43 ms).
+      starting_variant(v_exact::FusedLauncher<double, 16, 8, 256>::variant(FUSED_FP64_EXACT), 64.7),
+      starting_variant(v_exact::FusedLauncher<double, 8, 8, 256>::variant(FUSED_FP64_EXACT), 38.3),
       // the run-time solver kernel (HLLE / HLLC); not one of the tuned variants
-      v_exact::FusedLauncher<double, 32, 4, 128, 1, true>::variant(FUSED_FP64_EXACT),
+      v_exact::FusedLauncher<double, 16, 8, 256, 1, true>::variant(FUSED_FP64_EXACT),
   };
   *out = v;
   return (int)(sizeof(v) / sizeof(v[0])) - 1;  // the last entry is the run-time solver kernel
