@@ -801,19 +801,20 @@ k_fused_step(const InstanceDesc* __restrict__ desc, LaunchCtrl* __restrict__ lc)
   if (tid == 0) fused_finish_cta(desc, lc, ninst);
 }
 
-// Recovery of P from U for the interior (+ ghost images) and the dt/c_h reduction into slot: the
-// state a fused run starts from.  uh_in null: from the device U.  Otherwise the state comes from the caller's
+// Recovery of P from U for the interior (+ ghost images) and the dt/c_h reduction into the next step's slot:
+// the state a fused run starts from.  uh_in null: from the device U.  Otherwise the state comes from the caller's
 // host array (reference layout, itot x jtot x ktot, over the host link): every cell is copied into
 // the device U on the way, interior cells are recovered, and ghost cells also go to uh_ghost_out
 // when it is given (an output array other than the input).
 template <class R>
-__global__ void k_recover(FusedArgs a, int which, RedSlot* slot, const double* __restrict__ uh_in,
-                          double* __restrict__ uh_ghost_out) {
+__global__ void k_recover(FusedArgs a, const double* __restrict__ uh_in, double* __restrict__ uh_ghost_out) {
   __shared__ double scratch[64];
   const Layout L = a.L;
   R mn = R(1e30), mx = R(0);
   unsigned bad = 0;
-  R* Pout = reinterpret_cast<R*>(a.P[which]);
+  const unsigned long long step = a.ctrl->step;
+  RedSlot* slot = &a.ctrl->slot[step % 3];
+  R* Pout = reinterpret_cast<R*>(a.P[step & 1]);
   const long long stride = (long long)gridDim.x * blockDim.x;
   if (!uh_in) {
     const long long n = (long long)L.nx * L.ny * L.nz;
@@ -887,13 +888,13 @@ struct FusedLauncher {
 };
 
 template <class R>
-cudaError_t recover_launch(const FusedArgs& a, int which, RedSlot* slot, int nsm, cudaStream_t s,
+cudaError_t recover_launch(const FusedArgs& a, int nsm, cudaStream_t s,
                            const double* uh_in, double* uh_ghost_out) {
   const int bs = 256;
   const long long n = uh_in ? (long long)a.L.itot * a.L.jtot * a.L.ktot : (long long)a.L.nx * a.L.ny * a.L.nz;
   long long g = (n + bs - 1) / bs;
   if (g > (long long)nsm * 8) g = (long long)nsm * 8;
-  k_recover<R><<<(unsigned)g, bs, 0, s>>>(a, which, slot, uh_in, uh_ghost_out);
+  k_recover<R><<<(unsigned)g, bs, 0, s>>>(a, uh_in, uh_ghost_out);
   return cudaGetLastError();
 }
 

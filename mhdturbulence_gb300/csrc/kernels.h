@@ -20,7 +20,6 @@ cudaError_t launch_damp_psi(double* U, const Layout& L, const double* dxs, const
 cudaError_t launch_update_prim(const double* U, double* P, const Layout& L, double gam, cudaStream_t s);
 cudaError_t launch_reduce_dt_ch(const double* P, const Layout& L, const double* dxs, const double* dys,
                                 const double* dzs, RedSlot* slot, unsigned* status, int nsm, cudaStream_t s);
-cudaError_t launch_reset_slot(RedSlot* slot, cudaStream_t s);
 cudaError_t launch_slot_to_scalars(const RedSlot* slot, double cfl, double* dt, double* ch, cudaStream_t s);
 size_t pack_buffer_doubles(const Layout& L);
 cudaError_t launch_ghost_fill(double* P, const Layout& L, const int bc[6], double* scratch, cudaStream_t s);
@@ -37,20 +36,20 @@ int fused_variants(FusedKind kind, const FusedVariant** out);
 // The tile variant a grid starts with before any autotuning: the table entry marked preferred (the
 // fastest measured on GB300 at the benchmark sizes, 150^3 and 256^3).
 int fused_preferred_variant(FusedKind kind);
-// Recover P (FP64 for FP64 kinds, FP32 for mixed) + ghost images from a.U into a.P[which];
-// reduce dt/c_h into slot.
-cudaError_t launch_recover(FusedKind kind, const FusedArgs& a, int which, RedSlot* slot, int nsm, cudaStream_t s,
+// Recover P (FP64 for FP64 kinds, FP32 for mixed) + ghost images from a.U into the P buffer that the next step
+// reads; reduce that step's dt/c_h into its slot (both found from a.ctrl's step count on the device).
+cudaError_t launch_recover(FusedKind kind, const FusedArgs& a, int nsm, cudaStream_t s,
                            const double* uh_in = nullptr, double* uh_ghost_out = nullptr);
 
 namespace detail {
 int variants_exact(const FusedVariant** out);
 int variants_fp64(const FusedVariant** out);
 int variants_mixed(const FusedVariant** out);
-cudaError_t recover_exact(const FusedArgs& a, int which, RedSlot* slot, int nsm, cudaStream_t s, const double* uh_in,
+cudaError_t recover_exact(const FusedArgs& a, int nsm, cudaStream_t s, const double* uh_in,
                           double* uh_ghost_out);
-cudaError_t recover_fp64(const FusedArgs& a, int which, RedSlot* slot, int nsm, cudaStream_t s, const double* uh_in,
+cudaError_t recover_fp64(const FusedArgs& a, int nsm, cudaStream_t s, const double* uh_in,
                           double* uh_ghost_out);
-cudaError_t recover_mixed(const FusedArgs& a, int which, RedSlot* slot, int nsm, cudaStream_t s, const double* uh_in,
+cudaError_t recover_mixed(const FusedArgs& a, int nsm, cudaStream_t s, const double* uh_in,
                           double* uh_ghost_out);
 cudaError_t fdiv_selftest(int n, unsigned long long seed, unsigned long long* d_max_ulp, cudaStream_t s);
 }  // namespace detail

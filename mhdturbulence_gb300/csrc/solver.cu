@@ -93,6 +93,17 @@ __global__ void k_ctrl_restore(Ctrl* c, unsigned long long step, double time, do
   c->work_next = 0;
 }
 
+// Before a run: empty reduction slots for the next step and the one after it; with d, the step's host copy of U
+// (see k_set_host_u).
+__global__ void k_open_run(Ctrl* c, InstanceDesc* d, double* v) {
+  for (unsigned s = 0; s < 2; s++) {
+    RedSlot& r = c->slot[(c->step + s) % 3];
+    r.dtmin_bits = DT_RESET;
+    r.chmax_bits = CH_RESET;
+  }
+  if (d) d->a.Uh = v;
+}
+
 // Point the step's host copy of U at v (null: none), in the launch descriptor on the device.
 __global__ void k_set_host_u(InstanceDesc* d, double* v) { d->a.Uh = v; }
 
@@ -1217,15 +1228,12 @@ int mhdgb_prepare(mhdgb_solver* h) {
   int rc = set_device(h);
   if (rc) return rc;
   if (!h->have_state) return fail(h, MHDGB_ERR_STATE, "no state uploaded");
+  k_open_run<<<1, 1, 0, h->stream>>>(h->ctrl, nullptr, nullptr);
+  CK(h, cudaGetLastError());
+  CK(h, launch_recover(h->kind, fused_args(h), h->nsm, h->stream));
   Ctrl c;
   if ((rc = read_ctrl(h, &c))) return rc;
   h->cur_step = (long long)c.step;
-  const int cur = cur_index(h);
-  CK(h, launch_reset_slot(&h->ctrl->slot[c.step % 3], h->stream));
-  CK(h, launch_reset_slot(&h->ctrl->slot[(c.step + 1) % 3], h->stream));
-  FusedArgs a = fused_args(h);
-  CK(h, launch_recover(h->kind, a, cur, &h->ctrl->slot[c.step % 3], h->nsm, h->stream));
-  CK(h, cudaStreamSynchronize(h->stream));
   h->prepared = true;
   h->p64_valid = h->kind != FUSED_MIXED;
   return MHDGB_OK;
@@ -1319,20 +1327,20 @@ namespace {
 // the cells' accesses (rows of 16 or 32 values at 8-byte alignment) move more sectors than they use, so
 // U_in and U_out go through whole-sector repacking passes instead.  150^3: 4.03 -> 3.67 ms for a mixed
 // call; an FP64 call takes 5.22 ms as it is and 5.28 with a repacked U_in (1.43 ms and a recovery of
-// 0.25 after it, against 1.68 in one pass).
+// 0.25 after it, against 1.68 in one pass).  The P buffer and the slots follow from the step count on the
+// device, so nothing waits for the host to read it first (24x40x20 FP64 141 -> 124 us with the two launches
+// less).
 int step_host_mapped(mhdgb_solver* h, const double* din, double* dout, bool same, int nsteps) {
   const bool overlap = h->kind != FUSED_MIXED;
-  Ctrl c;
-  int rc = read_ctrl(h, &c);
-  if (rc) return rc;
-  h->cur_step = (long long)c.step;
+  int rc = MHDGB_OK;
   h->have_state = true;
   h->p_user = false;
   if (!overlap) CK(h, repack(din, h->U, h->L, NCONS, 1, h->nsm, h->stream));
-  CK(h, launch_reset_slot(&h->ctrl->slot[c.step % 3], h->stream));
-  CK(h, launch_reset_slot(&h->ctrl->slot[(c.step + 1) % 3], h->stream));
-  CK(h, launch_recover(h->kind, fused_args(h), cur_index(h), &h->ctrl->slot[c.step % 3], h->nsm, h->stream,
-                       overlap ? din : nullptr, overlap && !same ? dout : nullptr));
+  const bool one = overlap && nsteps == 1;
+  k_open_run<<<1, 1, 0, h->stream>>>(h->ctrl, one ? h->d_desc : nullptr, dout);
+  CK(h, cudaGetLastError());
+  CK(h, launch_recover(h->kind, fused_args(h), h->nsm, h->stream, overlap ? din : nullptr,
+                       overlap && !same ? dout : nullptr));
   h->prepared = true;
   h->p64_valid = h->kind != FUSED_MIXED;
   if (!overlap) {
@@ -1340,9 +1348,11 @@ int step_host_mapped(mhdgb_solver* h, const double* din, double* dout, bool same
     CK(h, repack(h->U, dout, h->L, NCONS, 0, h->nsm, h->stream));
     return MHDGB_OK;
   }
-  if (nsteps > 1 && (rc = mhdgb_step(h, nsteps - 1))) return rc;
-  k_set_host_u<<<1, 1, 0, h->stream>>>(h->d_desc, dout);
-  CK(h, cudaGetLastError());
+  if (!one) {
+    if ((rc = mhdgb_step(h, nsteps - 1))) return rc;
+    k_set_host_u<<<1, 1, 0, h->stream>>>(h->d_desc, dout);
+    CK(h, cudaGetLastError());
+  }
   rc = mhdgb_step(h, 1);
   k_set_host_u<<<1, 1, 0, h->stream>>>(h->d_desc, nullptr);
   CK(h, cudaGetLastError());
