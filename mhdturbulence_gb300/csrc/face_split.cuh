@@ -25,8 +25,8 @@
 // corrections enter as the innermost addend of the flux's last FMAs, and there are no branches before
 // the end, so that one face's conversions, pair chains and FP64 instructions overlap.
 //
-// Measured on the FP64 fused step (KH 150^3 / 256^3): 2.68 / 2.57 -> 1.09 / 1.02 ns per cell and step,
-// FP64-pipe instructions 1350 -> 394 per cell, with the limited slopes and the dt / c_h candidates below
+// Measured on the FP64 fused step (KH 150^3 / 256^3): 2.68 / 2.57 -> 1.08 / 1.01 ns per cell and step,
+// FP64-pipe instructions 1350 -> 393 per cell, with the limited slopes and the dt / c_h candidates below
 // in pairs too (1.27 / 1.21 with renormalised pairs, branches and two subtractions per slope).
 // Against the step in 64 bits the error over the Kelvin-Helmholtz, turbulence and smooth states at CFL
 // 0.05 and 0.3 is 0.46 to 1.04 times that of the FP64 expressions it replaced (geometric mean 0.86).

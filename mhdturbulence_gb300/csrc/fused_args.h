@@ -69,11 +69,12 @@ struct FusedVariant {
   int (*ctas_per_sm)();        // occupancy
   cudaError_t (*launch)(const InstanceDesc* desc, LaunchCtrl* lc, int grid, cudaStream_t s);
   const char* name;            // kernel form and tile shape, e.g. "two-phase 16x8/256"
-  int preferred;               // 1: the entry a grid starts on before any autotuning
+  int preferred;               // 1: the entry that grids of the benchmark sizes start on
   double plane_us;             // > 0: a smaller grid may start on this entry too; measured time of a full tile's plane
 };
 
-// Marks the table entry a grid starts on: the fastest measured on GB300 at the benchmark sizes.
+// Marks the table entry that grids of the benchmark sizes and ensembles start on (in FP64 and the mixed form the
+// fastest measured there on GB300).
 inline FusedVariant preferred_variant(FusedVariant v) {
   v.preferred = 1;
   return v;

@@ -33,8 +33,8 @@ cudaError_t launch_snapshot(const double* U, const double* P, const Layout& L, d
 // returns n, the number of HLLD tile variants out[0..n-1]; out[n] is the kind's run-time solver
 // kernel (HLLD, HLLE or HLLC from the arguments).
 int fused_variants(FusedKind kind, const FusedVariant** out);
-// The tile variant a grid starts with before any autotuning: the table entry marked preferred (the
-// fastest measured on GB300 at the benchmark sizes, 150^3 and 256^3).
+// The table entry marked preferred: what an ensemble, and a grid of the benchmark sizes (150^3 and 256^3) or
+// larger, starts with before any autotuning.
 int fused_preferred_variant(FusedKind kind);
 // Recover P (FP64 for FP64 kinds, FP32 for mixed) + ghost images from a.U into the P buffer that the next step
 // reads; reduce that step's dt/c_h into its slot (both found from a.ctrl's step count on the device).
