@@ -156,10 +156,15 @@ MHDGB_HD Pair p_narrow(double d) {
   const float l = f_mul(f_mul(i_to_f((int)(lo << 3)), 0x1p-32f), f_from(e | (hi & 0x80000000u)));
   return Pair{z ? 0.0f : d_round_f(hi, lo), z ? 0.0f : l};
 }
-// x / 2, x zero or normal and above 2^-1021.
+// x / 2 rounded to nearest even, for any x, on the integer pipe.  A front that decays into a uniform
+// background cell by cell passes through the subnormal numbers, so no magnitude is left out.
 MHDGB_HD double d_half(double x) {
-  const unsigned hi = d_hi(x);
-  return d_from((hi << 1) == 0u ? hi : hi - (1u << 20), d_lo(x));
+  const unsigned hi = d_hi(x), lo = d_lo(x), e = hi & 0x7FF00000u;
+  // exponent field 0 or 1: the magnitude is a whole number of the smallest subnormal
+  const unsigned sl = (hi << 31) | (lo >> 1), l = sl + ((lo & 3u) == 3u ? 1u : 0u);
+  const unsigned h = ((hi & 0x7FFFFFFFu) >> 1) + (l < sl ? 1u : 0u) + (hi & 0x80000000u);
+  const bool tiny = e < (2u << 20), keep = e == 0x7FF00000u;  // infinities and NaN stay
+  return d_from(tiny ? h : (keep ? hi : hi - (1u << 20)), tiny ? l : lo);
 }
 // h + l as a double (within an ulp), on the integer pipe, for a normalised pair; ex is added to the
 // result's high word (a power of two, given as its exponent << 20).  h = 0 gives 0.
