@@ -193,7 +193,7 @@ MHDGB_HD bool face_flux_split(const double (&Pl)[NPRIM], const double (&Pr)[NPRI
     e2 = p_fma(Dvz, p_fma(hq, v2z, bzst), e2);
     if (!nondeg) e2 = p_fma(p_sel(left, dl, dr), bx, e2);
     const Pair ab = f_bits(bx.h) >> 31 ? p_neg(bx) : bx;
-    const Pair S2 = p_sub(p_mul(ab, iq), sms);
+    const Pair S2 = p_norm(p_sub(p_mul(ab, iq), sms));  // normalised: its sign is that of h
     const Pair a2 = p_neg_if(S2.h > 0.0f ? S2 : p_make(0.0f), !left);
     const Pair ahq = p_mul(a2, hq);
     ce = p_sub(ce, p_mul(ahq, e2));

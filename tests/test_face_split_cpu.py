@@ -79,3 +79,108 @@ def test_subnormal_normal_field_and_psi(host, field, riemann):
         want = {5: lo, 8: -0.5 * CH * hi}
     for m, w in want.items():
         assert (np.abs(F[:, m] - w) <= 2.0 * np.spacing(np.abs(w))).all()
+
+
+def reference(left, right, riemann="hlld"):
+    """The flux (n, 10) of mhd.cpp:97-417 (with its energy flux term B^2 B_n, mhd.cpp:1049) in extended precision, and for each component the magnitudes of the terms it is the
+    sum of: the upwind side's physical flux, and wave speed times jump for each wave inside the fan."""
+    L, R = (np.asarray(a, dtype=np.longdouble).T for a in (left, right))
+
+    def side(P):
+        rho, vx, vy, vz, e, p, cs, bx, by, bz, psi, x = P
+        b2 = bx * bx + by * by + bz * bz
+        E = rho * e + rho * (vx * vx + vy * vy + vz * vz) / 2 + b2 / 2
+        pt = p + b2 / 2
+        U = [rho, rho * vx, rho * vy, rho * vz, E, by, bz, rho * x]
+        F = [[rho * vx], [rho * vx * vx, pt, -bx * bx], [rho * vy * vx, -by * bx], [rho * vz * vx, -bz * bx],
+             [E * vx, pt * vx, -b2 * bx], [by * vx, -vy * bx], [bz * vx, -vz * bx], [rho * x * vx]]
+        a = cs * cs + b2 / rho
+        cf = np.sqrt((a + np.sqrt((cs * cs - bx * bx / rho) ** 2 + (by * by + bz * bz) / rho *
+                                  (2 * cs * cs + 2 * bx * bx / rho + (by * by + bz * bz) / rho))) / 2)
+        return U, F, cf, pt
+
+    (Ul, Fl, cl, pl), (Ur, Fr, cr, pr) = side(L), side(R)
+    c = np.maximum(cl, cr)
+    vl, vr = L[VX], R[VX]
+    sl, sr = np.minimum(vl, vr) - c, np.maximum(vl, vr) + c
+    al, ar = L[DEN] * (sl - vl), R[DEN] * (sr - vr)
+    sm = (ar * vr - al * vl - pr + pl) / (ar - al)
+    ps = (ar * pl - al * pr + al * ar * (vr - vl)) / (ar - al)
+    bx = (L[BX] + R[BX]) / 2
+
+    def star(P, U, s, a, pt):
+        rho = a / (s - sm)
+        if riemann == "hllc":
+            k = rho / P[DEN]
+            return [rho, rho * sm, rho * P[VY], rho * P[VZ], ((s - P[VX]) * U[4] - pt * P[VX] + ps * sm) / (s - sm), k * U[5],
+                    k * U[6], k * U[7]], None
+        T = a * (s - sm) - bx * bx
+        t1, t2 = bx * (sm - P[VX]) / T, (a * (s - P[VX]) - bx * bx) / T
+        vy, vz, by, bz = P[VY] - P[BY] * t1, P[VZ] - P[BZ] * t1, P[BY] * t2, P[BZ] * t2
+        vb = sm * bx + vy * by + vz * bz
+        E = ((s - P[VX]) * U[4] - pt * P[VX] + ps * sm + bx * (P[VX] * bx + P[VY] * P[BY] + P[VZ] * P[BZ] - vb)) / (s - sm)
+        return [rho, rho * sm, rho * vy, rho * vz, E, by, bz, rho * P[X]], (vy, vz, vb)
+
+    (Sl, tl), (Sr, tr) = star(L, Ul, sl, al, pl), star(R, Ur, sr, ar, pr)
+    up = ~(sm < 0)
+    terms = [[np.where(up, p, q) for p, q in zip(f, g)] for f, g in zip(Fl, Fr)]
+    s = np.where(up, np.minimum(sl, 0), np.maximum(sr, 0))
+    for m in range(8):
+        terms[m].append(s * np.where(up, Sl[m] - Ul[m], Sr[m] - Ur[m]))
+    if riemann == "hlld":
+        ql, qr, h = np.sqrt(Sl[0]), np.sqrt(Sr[0]), np.where(bx < 0, -1, 1)
+        vy, vz = ((ql * a + qr * b + h * (q - p)) / (ql + qr) for a, b, p, q in
+                  ((tl[0], tr[0], Sl[5], Sr[5]), (tl[1], tr[1], Sl[6], Sr[6])))
+        by, bz = ((ql * q + qr * p + h * ql * qr * (b - a)) / (ql + qr) for a, b, p, q in
+                  ((tl[0], tr[0], Sl[5], Sr[5]), (tl[1], tr[1], Sl[6], Sr[6])))
+        vb = sm * bx + vy * by + vz * bz
+        q, i = np.where(up, ql, qr), np.where(up, 1, -1)
+        S = [np.where(up, a, b) for a, b in zip(Sl, Sr)]
+        s2 = np.where(up, np.minimum(sm - abs(bx) / ql, 0), np.maximum(sm + abs(bx) / qr, 0)) * (bx != 0)
+        dd = {2: S[0] * vy - S[2], 3: S[0] * vz - S[3], 4: -i * h * q * (np.where(up, tl[2], tr[2]) - vb), 5: by - S[5],
+              6: bz - S[6]}
+        for m, d in dd.items():
+            terms[m].append(s2 * d)
+    terms = terms[:5] + [[(L[PSI] + R[PSI]) / 2, -CH * (R[BX] - L[BX]) / 2]] + terms[5:7] + \
+        [[CH * CH * bx, -CH * (R[PSI] - L[PSI]) / 2], terms[7]]
+    return np.stack([sum(t) for t in terms], axis=1), np.stack([sum(abs(x) for x in t) for t in terms], axis=1)
+
+
+# A pair carries 48 bits, and the chains behind a correction lose a few of them: 2^-43 of the flux's terms is
+# the accuracy that the form states for itself.
+def assert_accurate(host, left, right, riemann, taken):
+    F, ok = faces(host, left, right, riemann)
+    assert ok.mean() >= taken
+    ref, scale = reference(left, right, riemann)
+    err = np.abs(F - ref) / np.where(scale > 0, scale, 1)
+    assert err[ok].max() <= 2.0 ** -43, (err[ok].max(axis=0), 2.0 ** -43)
+
+
+def _random(rng, n, **width):
+    """Background fields of order one, and a jump of the given width in each."""
+    mid = dict(rho=rng.uniform(0.5, 1.5, n), vx=rng.uniform(-0.8, 0.8, n), vy=rng.uniform(-0.8, 0.8, n), vz=rng.uniform(-0.8, 0.8, n),
+               p=rng.uniform(0.3, 1.5, n), bx=rng.uniform(-1, 1, n), by=rng.uniform(-1, 1, n), bz=rng.uniform(-1, 1, n),
+               psi=rng.uniform(-0.01, 0.01, n), X=rng.uniform(0, 1, n))
+    out = []
+    for _ in range(2):
+        out.append(states(n, **{k: v + width.get(k, width["all"]) * rng.uniform(-0.5, 0.5, n) for k, v in mid.items()}))
+    return out
+
+
+@pytest.mark.parametrize("riemann", ["hlld", "hllc"])
+@pytest.mark.parametrize("jump", [1e-12, 1e-6, 1e-2, 0.1])
+def test_accuracy_over_jumps(host, jump, riemann):
+    left, right = _random(np.random.default_rng(2), 20000, all=jump, psi=0.01 * jump)
+    assert_accurate(host, left, right, riemann, 0.5)
+
+
+def test_nearly_stationary_alfven_wave(host):
+    """S_M -+ |B_n| / sqrt(rho*) swept through zero: the rotation's flux is switched by the sign of a
+    difference that cancels."""
+    rng = np.random.default_rng(3)
+    n = 20000
+    rho, b, bt, th = rng.uniform(0.5, 1.5, n), rng.uniform(0.2, 1, n), rng.uniform(0.2, 1, n), rng.uniform(0, 2 * np.pi, n)
+    v = rng.choice([-1.0, 1.0], n) * b / np.sqrt(rho) * (1 + 10.0 ** rng.uniform(-16, -2, n) * rng.choice([-1.0, 1.0], n))
+    common = dict(rho=rho, vx=v, p=rng.uniform(0.3, 1.5, n), bx=b * rng.choice([-1.0, 1.0], n), X=0.5)
+    left, right = (states(n, by=bt * np.cos(a), bz=bt * np.sin(a), **common) for a in (th, th + rng.uniform(-0.02, 0.02, n)))
+    assert_accurate(host, left, right, "hlld", 0.9)
