@@ -76,7 +76,8 @@ MHDGB_HD bool face_flux_split(const double (&Pl)[NPRIM], const double (&Pr)[NPRI
   const Pair dvx = p_narrow(Pr[nve1] - Pl[nve1]);
   const Pair dby = p_narrow(Pr[nbm2] - Pl[nbm2]), dbz = p_narrow(Pr[nbm3] - Pl[nbm3]);
   const double jb = Pr[nbm1] - Pl[nbm1], hb = d_half(Pl[nbm1] + Pr[nbm1]);
-  const Pair dbx = p_narrow(jb), bxs = p_add(bxl, bxr), bx = p_scale(bxs, 0.5f);
+  // (B_n from the FP64 mean: a sum of the sides' pairs may cancel, and its h then has neither sign nor size)
+  const Pair dbx = p_narrow(jb), bx = p_narrow(hb), bxs = p_scale(bx, 2.0f);
 
   // fast speeds: c_f^2 = (a + b + sqrt((a-b)^2 + t (t + 2(a+b)))) / 2 with a = c_s^2, b = B_n^2/rho,
   // t = B_t^2/rho (the discriminant as a sum of squares, without cancellation)

@@ -83,7 +83,9 @@ def test_subnormal_normal_field_and_psi(host, field, riemann):
 
 def reference(left, right, riemann="hlld"):
     """The flux (n, 10) of mhd.cpp:97-417 (with its energy flux term B^2 B_n, mhd.cpp:1049) in extended precision, and for each component the magnitudes of the terms it is the
-    sum of: the upwind side's physical flux, and wave speed times jump for each wave inside the fan."""
+    sum of: the upwind side's physical flux, and wave speed times jump for each wave inside the fan, a speed or
+    a jump that is itself a difference of larger terms (jumps of velocity and pressure; S_M and |B_n| / sqrt(rho*))
+    counted by those."""
     L, R = (np.asarray(a, dtype=np.longdouble).T for a in (left, right))
 
     def side(P):
@@ -104,7 +106,8 @@ def reference(left, right, riemann="hlld"):
     vl, vr = L[VX], R[VX]
     sl, sr = np.minimum(vl, vr) - c, np.maximum(vl, vr) + c
     al, ar = L[DEN] * (sl - vl), R[DEN] * (sr - vr)
-    sm = (ar * vr - al * vl - pr + pl) / (ar - al)
+    dpt = R[PRE] - L[PRE] + sum((R[q] - L[q]) * (R[q] + L[q]) for q in (BX, BY, BZ)) / 2  # (pr - pl would round)
+    sm = (ar * vr - al * vl - dpt) / (ar - al)
     ps = (ar * pl - al * pr + al * ar * (vr - vl)) / (ar - al)
     bx = (L[BX] + R[BX]) / 2
 
@@ -124,9 +127,22 @@ def reference(left, right, riemann="hlld"):
     (Sl, tl), (Sr, tr) = star(L, Ul, sl, al, pl), star(R, Ur, sr, ar, pr)
     up = ~(sm < 0)
     terms = [[np.where(up, p, q) for p, q in zip(f, g)] for f, g in zip(Fl, Fr)]
+    size = [[abs(x) for x in t] for t in terms]
+    # S_M relative to a side: (rho_o (v_r - v_l) -+ (pt_r - pt_l) / w) / (rho_l + rho_r)
+    w = c - np.minimum(vr - vl, 0)
+    # (the mean of B_n is one FP64 sum; those of B_t are sums of pairs)
+    psize = abs(R[PRE] - L[PRE]) + (abs((R[BX] - L[BX]) * (R[BX] + L[BX])) +
+                                    sum(abs(R[q] - L[q]) * (abs(R[q]) + abs(L[q])) for q in (BY, BZ))) / 2
+    d = abs(sm - np.where(up, vl, vr))
+    dsize = (np.where(up, R[DEN], L[DEN]) * abs(vr - vl) + psize / w) / (L[DEN] + R[DEN])
+    grow = np.where(d > 0, dsize / np.where(d > 0, d, 1), 1)
     s = np.where(up, np.minimum(sl, 0), np.maximum(sr, 0))
+    jump = [np.where(up, a - b, e - f) for a, b, e, f in zip(Sl, Ul, Sr, Ur)]
+    jump[0] = np.where(up, L[DEN] * (sm - vl) / (sl - sm), R[DEN] * (sm - vr) / (sr - sm))  # (rho* - rho would round)
+    jump[7] = jump[0] * np.where(up, L[X], R[X])
     for m in range(8):
-        terms[m].append(s * np.where(up, Sl[m] - Ul[m], Sr[m] - Ur[m]))
+        terms[m].append(s * jump[m])
+        size[m].append(abs(terms[m][-1]) * grow)
     if riemann == "hlld":
         ql, qr, h = np.sqrt(Sl[0]), np.sqrt(Sr[0]), np.where(bx < 0, -1, 1)
         vy, vz = ((ql * a + qr * b + h * (q - p)) / (ql + qr) for a, b, p, q in
@@ -139,11 +155,20 @@ def reference(left, right, riemann="hlld"):
         s2 = np.where(up, np.minimum(sm - abs(bx) / ql, 0), np.maximum(sm + abs(bx) / qr, 0)) * (bx != 0)
         dd = {2: S[0] * vy - S[2], 3: S[0] * vz - S[3], 4: -i * h * q * (np.where(up, tl[2], tr[2]) - vb), 5: by - S[5],
               6: bz - S[6]}
-        for m, d in dd.items():
-            terms[m].append(s2 * d)
-    terms = terms[:5] + [[(L[PSI] + R[PSI]) / 2, -CH * (R[BX] - L[BX]) / 2]] + terms[5:7] + \
-        [[CH * CH * bx, -CH * (R[PSI] - L[PSI]) / 2], terms[7]]
-    return np.stack([sum(t) for t in terms], axis=1), np.stack([sum(abs(x) for x in t) for t in terms], axis=1)
+        qo = np.where(up, qr, ql)
+        D = [(qo * (abs(tl[a] - L[v]) + abs(tr[a] - R[v]) + abs(R[v] - L[v])) +
+              abs(Sl[b] - L[f]) + abs(Sr[b] - R[f]) + abs(R[f] - L[f])) / (ql + qr)
+             for a, v, b, f in ((0, VY, 5, BY), (1, VZ, 6, BZ))]
+        s2size = (s2 != 0) * (abs(sm) + abs(bx) / q)
+        dsizes = {2: S[0] * D[0], 3: S[0] * D[1], 5: q * D[0], 6: q * D[1],
+                  4: q * (D[0] * (abs(S[5]) + q * abs(vy)) + D[1] * (abs(S[6]) + q * abs(vz)))}
+        for m, e in dd.items():
+            terms[m].append(s2 * e)
+            size[m].append(s2size * dsizes[m])
+    glm = [[(L[PSI] + R[PSI]) / 2, -CH * (R[BX] - L[BX]) / 2], [CH * CH * bx, -CH * (R[PSI] - L[PSI]) / 2]]
+    glms = [[(abs(L[PSI]) + abs(R[PSI])) / 2, abs(glm[0][1])], [CH * CH * (abs(L[BX]) + abs(R[BX])) / 2, abs(glm[1][1])]]
+    terms, size = (x[:5] + [g[0]] + x[5:7] + [g[1], x[7]] for x, g in ((terms, glm), (size, glms)))
+    return np.stack([sum(t) for t in terms], axis=1), np.stack([sum(t) for t in size], axis=1)
 
 
 # A pair carries 48 bits, and the chains behind a correction lose a few of them: 2^-43 of the flux's terms is
@@ -183,4 +208,15 @@ def test_nearly_stationary_alfven_wave(host):
     v = rng.choice([-1.0, 1.0], n) * b / np.sqrt(rho) * (1 + 10.0 ** rng.uniform(-16, -2, n) * rng.choice([-1.0, 1.0], n))
     common = dict(rho=rho, vx=v, p=rng.uniform(0.3, 1.5, n), bx=b * rng.choice([-1.0, 1.0], n), X=0.5)
     left, right = (states(n, by=bt * np.cos(a), bz=bt * np.sin(a), **common) for a in (th, th + rng.uniform(-0.02, 0.02, n)))
+    assert_accurate(host, left, right, "hlld", 0.9)
+
+
+def test_normal_fields_that_cancel(host):
+    """B_n of the two sides nearly opposite: the sign and size of their mean come from what is left."""
+    rng = np.random.default_rng(4)
+    n = 20000
+    b, by, bz = rng.uniform(0.2, 1, n), rng.uniform(-1, 1, n), rng.uniform(-1, 1, n)
+    left, right = (states(n, rho=rng.uniform(0.9, 1.1, n), vx=rng.uniform(-1e-9, 1e-9, n), vy=rng.uniform(-0.01, 0.01, n),
+                          vz=rng.uniform(-0.01, 0.01, n), p=1.0, bx=x, by=by + rng.uniform(-0.01, 0.01, n), bz=bz)
+                   for x in (b, -b * (1 + 10.0 ** rng.uniform(-16, -6, n) * rng.choice([-1.0, 1.0], n))))
     assert_accurate(host, left, right, "hlld", 0.9)
