@@ -106,7 +106,9 @@ MHDGB_HD bool face_flux_split(const double (&Pl)[NPRIM], const double (&Pr)[NPRI
   const Pair sm = p_mul(p_sub(p_fma(rr, vxr, p_mul(rl, vxl)), dpw), ir);
   const bool left = !(f_add(sm.h, sm.l) < 0.0f);
   const Pair dl = p_norm(p_mul(p_norm(p_sub(p_mul(rr, dvx), dpw)), ir));
-  const Pair dr = p_sub(dl, dvx);
+  // (dr formed as dl is, not as dl - dvx: with the right side much the denser that difference cancels, and
+  // mirror-image states would not give mirror-image fluxes)
+  const Pair dr = p_norm(p_mul(p_norm(p_neg(p_add(p_mul(rl, dvx), dpw))), ir));
 
   // upwind side; signs as seen from it (x_: times +1 on the left, -1 on the right)
   const double rho = left ? Pl[nden] : Pr[nden], vx = left ? Pl[nve1] : Pr[nve1], vy = left ? Pl[nve2] : Pr[nve2],

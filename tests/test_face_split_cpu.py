@@ -220,3 +220,31 @@ def test_normal_fields_that_cancel(host):
                           vz=rng.uniform(-0.01, 0.01, n), p=1.0, bx=x, by=by + rng.uniform(-0.01, 0.01, n), bz=bz)
                    for x in (b, -b * (1 + 10.0 ** rng.uniform(-16, -6, n) * rng.choice([-1.0, 1.0], n))))
     assert_accurate(host, left, right, "hlld", 0.9)
+
+
+def _mirrored(P):
+    M = P.copy()
+    M[:, [VX, BX]] *= -1.0
+    return M
+
+
+@pytest.mark.parametrize("riemann", ["hlld", "hllc"])
+@pytest.mark.parametrize("ratio", [1.0, 10.0, 1e3, 1e6])
+def test_mirror_images_and_density_ratios(host, ratio, riemann):
+    """Swapping the sides and mirroring the normal axis mirrors the flux bit for bit, whichever side is
+    the denser, and the flux keeps its accuracy on both."""
+    rng = np.random.default_rng(5)
+    left, right = _random(rng, 20000, all=0.1, bx=0.0, psi=0.001)
+    for P, k in ((left, 1.0), (right, ratio)):
+        P[:, DEN] *= k
+        P[:, ENE] /= k
+        P[:, CS] = np.sqrt(GAM * P[:, PRE] / P[:, DEN])
+    for a, b in ((left, right), (right, left)):
+        F, ok = faces(host, a, b, riemann)
+        G, ok2 = faces(host, _mirrored(b), _mirrored(a), riemann)
+        moving = F[:, 0] != 0  # (at S_M = 0 both take the left side)
+        sign = np.array([-1, 1, -1, -1, -1, 1, -1, -1, -1, -1.0])
+        assert np.array_equal(ok, ok2) and ok.any()
+        both = ok & moving
+        assert np.array_equal(F[both], (G * sign)[both])
+        assert_accurate(host, a, b, riemann, 0.2)
