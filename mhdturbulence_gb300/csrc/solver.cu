@@ -1334,13 +1334,16 @@ int step_host_mapped(mhdgb_solver* h, const double* din, double* dout, bool same
   const bool overlap = h->kind != FUSED_MIXED;
   int rc = MHDGB_OK;
   h->have_state = true;
+  h->prepared = false;  // until the recovery below has been launched
   h->p_user = false;
   if (!overlap) CK(h, repack(din, h->U, h->L, NCONS, 1, h->nsm, h->stream));
   const bool one = overlap && nsteps == 1;
   k_open_run<<<1, 1, 0, h->stream>>>(h->ctrl, one ? h->d_desc : nullptr, dout);
   CK(h, cudaGetLastError());
-  CK(h, launch_recover(h->kind, fused_args(h), h->nsm, h->stream, overlap ? din : nullptr,
-                       overlap && !same ? dout : nullptr));
+  const cudaError_t rec = launch_recover(h->kind, fused_args(h), h->nsm, h->stream, overlap ? din : nullptr,
+                                         overlap && !same ? dout : nullptr);
+  if (rec != cudaSuccess && one) k_set_host_u<<<1, 1, 0, h->stream>>>(h->d_desc, nullptr);  // no later step may write U_out
+  CK(h, rec);
   h->prepared = true;
   h->p64_valid = h->kind != FUSED_MIXED;
   if (!overlap) {
