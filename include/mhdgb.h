@@ -174,7 +174,8 @@ int mhdgb_reset_clock(mhdgb_solver* h);
  * host link (FP64 forms: the recovery pass reads U_in and the last step writes each updated cell of
  * U_out; mixed form: repacking passes before and after), and the ghost cells of a separate U_out are
  * U_in's.  Other arrays go through a device staging
- * buffer.  Both give the same U_out bit for bit; U_out may be U_in. */
+ * buffer.  Both give the same U_out bit for bit; U_out may be U_in.  Steps after the stop condition are
+ * skipped, as in mhdgb_step: U_out is then the state at the stop. */
 int mhdgb_step_host(mhdgb_solver* h, const double* U_in, double* U_out, int nsteps, double* dt, double* chg);
 
 /* Time nsteps fused steps with CUDA events recorded on the handle's stream around the enqueued

@@ -1377,7 +1377,8 @@ int mhdgb_step_host(mhdgb_solver* h, const double* U_in, double* U_out, int nste
   // arrays that overlap without being the same one take the staged route: the recovery pass writes
   // U_out's ghost cells while it is still reading U_in
   const bool partial_overlap = U_in != U_out && U_in < U_out + n && U_out < U_in + n;
-  if (din && dout && !partial_overlap) {
+  const bool mapped = din && dout && !partial_overlap;
+  if (mapped) {
     if ((rc = step_host_mapped(h, din, const_cast<double*>(dout), din == dout, nsteps))) return rc;
   } else {
     if ((rc = settle(h)) || (rc = upload_u(h, U_in))) return rc;
@@ -1387,8 +1388,14 @@ int mhdgb_step_host(mhdgb_solver* h, const double* U_in, double* U_out, int nste
     if ((rc = mhdgb_prepare(h)) || (rc = mhdgb_step(h, nsteps))) return rc;
     if ((rc = settle(h)) || (rc = download_u(h, U_out))) return rc;
   }
-  mhdgb_report rep;
+  mhdgb_report rep{};
   rc = mhdgb_sync(h, &rep);
+  // With the stop condition reached the last step may have been skipped, and with it the cells that it writes to a
+  // page-locked U_out; the state at the stop is on the device.
+  if (mapped && rep.done && h->kind != FUSED_MIXED) {
+    CK(h, repack(h->U, const_cast<double*>(dout), L, NCONS, 0, h->nsm, h->stream));
+    CK(h, cudaStreamSynchronize(h->stream));
+  }
   if (dt) *dt = rep.dt;
   if (chg) *chg = rep.chg;
   return rc;
