@@ -57,6 +57,22 @@ constexpr float kJump = 0.04f;
 
 MHDGB_HD unsigned d_mag(double d) { return d_hi(d) & 0x7FFFFFFFu; }
 
+// Whether the states of a face lie within the bounds.
+MHDGB_HD bool face_in_range(const double (&Pl)[NPRIM], const double (&Pr)[NPRIM]) {
+  unsigned mb = 0;
+#pragma unroll
+  for (int n = nbm2; n <= nbm3; n++) mb = u_max(mb, u_max(d_mag(Pl[n]), d_mag(Pr[n])));
+  unsigned mx = mb;
+  const int q[] = {nve1, nve2, nve3, nbm1, nden, ncsp};
+#pragma unroll
+  for (int n = 0; n < 6; n++) mx = u_max(mx, u_max(d_mag(Pl[q[n]]), d_mag(Pr[q[n]])));
+  // signed comparison: a negative value fails
+  const int mn = (int)kSplitMin;
+  const bool pos = (int)d_hi(Pl[nden]) >= mn && (int)d_hi(Pr[nden]) >= mn && (int)d_hi(Pl[ncsp]) >= mn &&
+                   (int)d_hi(Pr[ncsp]) >= mn;
+  return mx < kSplitMax && mb - 1u >= kSplitTinyB - 1u && pos;  // (mb = 0 passes)
+}
+
 // Flux through a face from its reconstructed states (rotated: normal component first), HLLD or, with
 // hllc, HLLC; returns false where the split does not apply (F is then meaningless).  hchg = c_h / 2, chg2 =
 // c_h^2 (the GLM pair, mhd.cpp:1234-1237).  The energy and the scalar are wanted on the upwind side only:
@@ -64,21 +80,8 @@ MHDGB_HD unsigned d_mag(double d) { return d_hi(d) & 0x7FFFFFFFu; }
 template <class UP>
 MHDGB_HD bool face_flux_split(const double (&Pl)[NPRIM], const double (&Pr)[NPRIM], const UP& up, double hchg,
                               double chg2, double (&F)[NCONS], bool hllc) {
-  bool ok;  // (checked at the end: a branch here would keep the loads and conversions below from overlapping)
-  {
-    unsigned mb = 0;
-#pragma unroll
-    for (int n = nbm2; n <= nbm3; n++) mb = u_max(mb, u_max(d_mag(Pl[n]), d_mag(Pr[n])));
-    unsigned mx = mb;
-    const int q[] = {nve1, nve2, nve3, nbm1, nden, ncsp};
-#pragma unroll
-    for (int n = 0; n < 6; n++) mx = u_max(mx, u_max(d_mag(Pl[q[n]]), d_mag(Pr[q[n]])));
-    // signed comparison: a negative value fails
-    const int mn = (int)kSplitMin;
-    const bool pos = (int)d_hi(Pl[nden]) >= mn && (int)d_hi(Pr[nden]) >= mn && (int)d_hi(Pl[ncsp]) >= mn &&
-                     (int)d_hi(Pr[ncsp]) >= mn;
-    ok = mx < kSplitMax && mb - 1u >= kSplitTinyB - 1u && pos;  // (mb = 0 passes)
-  }
+  // (checked at the end: a branch here would keep the loads and conversions below from overlapping)
+  bool ok = face_in_range(Pl, Pr);
   const Pair rl = p_narrow_nz(Pl[nden]), rr = p_narrow_nz(Pr[nden]);
   const Pair bxl = p_narrow(Pl[nbm1]), bxr = p_narrow(Pr[nbm1]);
   const Pair byl = p_narrow(Pl[nbm2]), byr = p_narrow(Pr[nbm2]);
