@@ -199,7 +199,9 @@ int mhdgb_work_layout(const mhdgb_solver* h, int* ntx, int* nty, int* nchunks, i
 /* The z chunking that the fused step plans for an nx x ny x nz grid cut into tx x ty tiles, on a
  * persistent launch of ctas CTAs: the host-side planner that mhdgb_work_layout reports the result
  * of (uniform, shrinking and geometric chunkings; the one whose simulated work queue finishes
- * first).  Writes the chunk lengths in planes (they sum to nz) to chunks[0 .. max_chunks) and
+ * first), for a kernel with more warps than its tile's columns need, as every kernel that a grid starts
+ * on has but the separately rounded form's 32x4/128 (whose own plan mhdgb_work_layout reports).
+ * Writes the chunk lengths in planes (they sum to nz) to chunks[0 .. max_chunks) and
  * returns their number, or MHDGB_ERR_ARG for a bad size or too small an array.  Needs no device. */
 int mhdgb_plan_zchunks(int nx, int ny, int nz, int tx, int ty, int ctas, int* chunks, int max_chunks);
 /* Time every compiled tile shape on the handle's grid (steps fused steps each, from the current

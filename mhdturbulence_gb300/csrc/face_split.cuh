@@ -7,7 +7,8 @@
 // about 2^-43, so they are formed from pairs of FP32 values (fp32pair.cuh, about 2^-46) on pipes that
 // are otherwise idle.  Each is written in the small quantities that drive it (the contact speed
 // relative to the side, the jumps), never as a difference of two nearly equal states, so its
-// relative accuracy carries over to the flux however small the jump is:
+// relative accuracy carries over to the flux however small the jump is; strong jumps take the general FP64
+// flux (kJump):
 //
 //   w  = max(c_f) + max(0, v_l - v_r)        the outer waves run at v_l - w and v_r + w
 //   d  = S_M - v                             from the jumps of v and of the total pressure
@@ -25,11 +26,12 @@
 // corrections enter as the innermost addend of the flux's last FMAs, and there are no branches before
 // the end, so that one face's conversions, pair chains and FP64 instructions overlap.
 //
-// Measured on the FP64 fused step (KH 150^3 / 256^3): 2.68 / 2.57 -> 1.08 / 1.01 ns per cell and step,
+// Measured on the FP64 fused step (KH 150^3 / 256^3): 2.68 / 2.57 -> 1.09 / 1.02 ns per cell and step,
 // FP64-pipe instructions 1350 -> 393 per cell, with the limited slopes and the dt / c_h candidates below
-// in pairs too (1.27 / 1.21 with renormalised pairs, branches and two subtractions per slope).
+// in pairs too (1.27 / 1.21 with renormalised pairs, branches and two subtractions per slope; 1.08 / 1.01 without
+// kJump's bounds and with the contact's and the Alfven waves' speeds from unnormalised differences).
 // Against the step in 64 bits the error over the Kelvin-Helmholtz, turbulence and smooth states at CFL
-// 0.05 and 0.3 is 0.46 to 1.04 times that of the FP64 expressions it replaced (geometric mean 0.86).
+// 0.05 and 0.3 is 0.41 to 1.02 times that of the FP64 expressions it replaced (geometric mean 0.79).
 #pragma once
 
 #include "fp32pair.cuh"
@@ -40,19 +42,22 @@ namespace mhdgb {
 // Bounds within which the pairs neither overflow nor lose their low parts: density and sound speed
 // in [2^-20, 2^20], velocities and fields below 2^20, the larger tangential field component zero or
 // above 2^-83 (pressure and energy follow from density and sound speed; a NaN in them is one in the
-// sound speed).  Other
-// faces take the general FP64 flux.
+// sound speed).  Other faces take the general FP64 flux.
 constexpr unsigned kSplitMax = (1023u + 20u) << 20, kSplitMin = (1023u - 20u) << 20, kSplitTinyB = (1023u - 83u) << 20;
 
 // Jumps beyond which the general flux is the more accurate one.  A correction's error is 2^-46 of the wave speed
 // times the jump that drives it, the FP64 expressions' a few 2^-53 of the fluxes' own terms, so the jumps are
 // bounded by 0.04: S_M relative to the sides and the rotations' velocity jump in units of w, each field
-// component's part of the magnetic pressure's jump in units of rho w^2 (the gas pressure may balance it).  (No outer wave comes near the contact then.)
+// component's part of the magnetic pressure's jump in units of rho w^2 (the gas pressure may balance it).  No outer
+// wave comes near the contact then.  (A tangential velocity's jump, the shear of a layer without B_n, is not bounded:
+// no wave carries it.)
 // Against extended precision the mean error of every flux component is then at most 1.1 times the FP64 expressions'
 // (0.2 to 0.9 times for jumps up to 0.1) over random states with jumps of 1e-6 to 1, pressure-balanced sheets,
 // low beta (1e-3), density ratios up to 2^16, stationary Alfven waves and reflecting walls.  Without the bounds it is 2.7
 // times for jumps of order one, 6 to 16 times at walls, whose mass flux is the difference of two such terms, and
-// 17 times for strong stationary rotations.
+// 17 times for strong stationary rotations.  A warp with such a face forms both fluxes: a smooth 24x40x20 state whose
+// walls start with a normal velocity takes 160 us a call instead of 124 (224 with FP64 expressions alone), decaying
+// turbulence of 128^3 at Mach 0.6 after 200 steps 1.19 ns a cell instead of 1.12 (2.62).
 constexpr float kJump = 0.04f;
 
 MHDGB_HD unsigned d_mag(double d) { return d_hi(d) & 0x7FFFFFFFu; }

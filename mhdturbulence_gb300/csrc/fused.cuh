@@ -674,8 +674,8 @@ k_fused_step(const InstanceDesc* __restrict__ desc, LaunchCtrl* __restrict__ lc)
           };
           if constexpr (kFast && std::is_same<R, double>::value) {
             // A thread whose last face of the general flux lay outside the pairs' range tests the range before the
-            // split, so that states wholly outside it (CGS units) do not pay for both: KH 150^3 there 11.2 -> 9.03 ms
-            // a step (8.95 with the FP64 expressions alone), and 3.68 -> 3.67 inside the range.
+            // split, so that states wholly outside it (CGS units) do not pay for both: KH 150^3 there 11.2 -> 9.04 ms
+            // a step (8.95 with the FP64 expressions alone), and 3.69 -> 3.68 inside the range.
             const bool hlle = GEN && riemann == RIEMANN_HLLE;
             bool done = false;
             auto general = [&]() {

@@ -238,10 +238,6 @@ __device__ __forceinline__ double twice_div_est(double p, double s) {
   return p * fma(h, fma(-s, y0, 2.0), y0);
 }
 
-// vanLeer, src_cpp_kokkos_host/mhd.cpp:89-95.  The limited slope of a cell c is
-// van_leer(P[c+1]-P[c], P[c]-P[c-1]); the reference evaluates the same expression for the left
-// state of face c+1/2 and the right state of face c-1/2 (mhd.cpp:1134-1154), so one evaluation
-// per cell and direction gives both.
 // 2 a b rounded as (2 a) b, from p = a b > 0: twice p unless p is subnormal or twice it overflows.
 __device__ __forceinline__ double twice_product(double p, double a, double b) {
   const unsigned e = (unsigned)__double2hiint(p) >> 20;
@@ -252,6 +248,10 @@ __device__ __noinline__ double van_leer_general(double dsvp, double dsvm) {
   const double p = dsvp * dsvm;
   return pos_nonzero(p) ? twice_div_est(p, dsvp + dsvm) : 0.0;
 }
+// vanLeer, src_cpp_kokkos_host/mhd.cpp:89-95.  The limited slope of a cell c is
+// van_leer(P[c+1]-P[c], P[c]-P[c-1]); the reference evaluates the same expression for the left
+// state of face c+1/2 and the right state of face c-1/2 (mhd.cpp:1134-1154), so one evaluation
+// per cell and direction gives both.
 template <class R>
 __device__ __forceinline__ R van_leer(R dsvp, R dsvm) {
   if constexpr (kFast) {  // one product for the test and the numerator: p + p == (2 dsvp) dsvm exactly

@@ -737,8 +737,8 @@ int use_variant(mhdgb_solver* h, int idx, int kc_fixed = 0, const std::vector<in
 // Smaller grids take the marked entry whose simulated queue finishes first, if it saves 5 %: few planes per
 // SM make the tile's share of idle threads and the number of rounds decide.  Simulated times are within 10 %
 // of the measured ones for 21 grids from 16^3 to 150^3 (8x8 tiles one cell wide: 25 % low); the picks were the
-// fastest entry or within 1 % of it but for 24^3 in the exact form (5 %).  All entries of a form give the same
-// result bit for bit.
+// fastest entry or within 1 % of it but for 24^3 in the exact form (5 %).  All entries of these two forms
+// give the same result bit for bit.
 // *plan receives the picked entry's chunks if they were simulated.
 int start_variant(const mhdgb_solver* h, std::vector<int>* plan) {
   const int pref = fused_preferred_variant(h->kind);
