@@ -46,18 +46,21 @@ namespace mhdgb {
 constexpr unsigned kSplitMax = (1023u + 20u) << 20, kSplitMin = (1023u - 20u) << 20, kSplitTinyB = (1023u - 83u) << 20;
 
 // Jumps beyond which the general flux is the more accurate one.  A correction's error is 2^-46 of the wave speed
-// times the jump that drives it, the FP64 expressions' a few 2^-53 of the fluxes' own terms, so the jumps are
-// bounded by 0.04: S_M relative to the sides and the rotations' velocity jump in units of w, each field
-// component's part of the magnetic pressure's jump in units of rho w^2 (the gas pressure may balance it).  No outer
-// wave comes near the contact then.  (A tangential velocity's jump, the shear of a layer without B_n, is not bounded:
-// no wave carries it.)
-// Against extended precision the mean error of every flux component is then at most 1.1 times the FP64 expressions'
-// (0.2 to 0.9 times for jumps up to 0.1) over random states with jumps of 1e-6 to 1, pressure-balanced sheets,
-// low beta (1e-3), density ratios up to 2^16, stationary Alfven waves and reflecting walls.  Without the bounds it is 2.7
-// times for jumps of order one, 6 to 16 times at walls, whose mass flux is the difference of two such terms, and
-// 17 times for strong stationary rotations.  A warp with such a face forms both fluxes: a smooth 24x40x20 state whose
-// walls start with a normal velocity takes 160 us a call instead of 124 (224 with FP64 expressions alone), decaying
-// turbulence of 128^3 at Mach 0.6 after 200 steps 1.19 ns a cell instead of 1.12 (2.62).
+// times the jump that drives it; the FP64 expressions' are a few 2^-53 of the fluxes' own terms, and 2^-43 (their
+// estimate of the fast speed) of what the outer waves carry with S_M.  So the bounds, in units of w:
+//   S_M relative to the sides, unless S_M itself is above 1/8 (a moving shock, not a wall),
+//   the rotations' velocity jump, times S_M or |B_n| / sqrt(rho*) where these are below 1/4 (without B_n a shear is
+//   no rotation's jump),
+//   and each field component's part of the magnetic pressure's jump, of rho w^2: the gas pressure may balance it.
+// No outer wave comes near the contact then.  Against extended precision the mean error of the flux components
+// from given face states is at most 1.15 times the FP64 expressions' (0.2 to 0.9 times for jumps up to 0.1; 1.2 times
+// where both only round FP64's last bit) over random states with jumps of 1e-6 to 1, pressure-balanced sheets, shears,
+// low beta (1e-3), density ratios up to 2^16, stationary Alfven waves and walls with a normal velocity; from cell
+// values, with the slopes' errors in it, 0.1 to 1.05 times.  Without the bounds it is up to 2.7 times for jumps of order
+// one, 17 times for strong stationary rotations and 8 to 16 times at walls, whose mass flux is the difference of two
+// such terms; from cell values the walls alone are worse than FP64 was.  A warp with such a face forms both fluxes: a
+// 24x40x20 state whose walls start with a normal velocity takes 161 us a call instead of 124 (224 with FP64
+// expressions alone), decaying turbulence of 128^3 at Mach 0.6 after 200 steps 1.14 ns a cell instead of 1.06 (2.62).
 constexpr float kJump = 0.04f;
 
 MHDGB_HD unsigned d_mag(double d) { return d_hi(d) & 0x7FFFFFFFu; }
@@ -145,7 +148,9 @@ MHDGB_HD bool face_flux_split(const double (&Pl)[NPRIM], const double (&Pr)[NPRI
   const Pair sms = p_neg_if(sm, !left), vs = p_neg_if(p_sel(left, vxl, vxr), !left), bs = p_neg_if(bx, !left);
   const Pair tauo = p_neg_if(p_sel(left, dr, dl), left);
   const Pair wmo = p_norm(p_add(w, tauo));
-  ok = ok && fmaxf(fabsf(dl.h), fabsf(dr.h)) < kJump * w.h && jump_b < 0.5f * kJump * f_add(rl.h, rr.h) * w.h * w.h;
+  const float d = fmaxf(fabsf(dl.h), fabsf(dr.h));
+  ok = ok && (d < kJump * w.h || (fabsf(sm.h) > 0.125f * w.h && d < 0.5f * w.h)) &&
+       jump_b < 0.5f * kJump * f_add(rl.h, rr.h) * w.h * w.h;
 
   const Pair iwm = p_rcp(wm);
   // T = N + rho w tau with N = rho w^2 - B_n^2 in FP64: near B_t = 0 the fast speed is close to the
@@ -208,7 +213,6 @@ MHDGB_HD bool face_flux_split(const double (&Pl)[NPRIM], const double (&Pr)[NPRI
     const Pair jbz = p_sub(p_fma(go, bzo, p_neg_if(dbz, !left)), gbz);
     const Pair Dvy = p_mul(p_fma(qo, jvy, p_neg_if(jby, hn)), inv);
     const Pair Dvz = p_mul(p_fma(qo, jvz, p_neg_if(jbz, hn)), inv);
-    ok = ok && fmaxf(fabsf(Dvy.h), fabsf(Dvz.h)) < kJump * w.h;
     const Pair hq = p_neg_if(q, hn);
     // E** - E* = h sqrt(rho*) (v**.B** - v*.B*) = h sqrt(rho*) sum Dv (B* + h sqrt(rho*) v**)
     const Pair v2y = p_add(p_add(vyu, fby), Dvy), v2z = p_add(p_add(vzu, fbz), Dvz);
@@ -217,6 +221,8 @@ MHDGB_HD bool face_flux_split(const double (&Pl)[NPRIM], const double (&Pr)[NPRI
     if (!nondeg) e2 = p_fma(p_sel(left, dl, dr), bx, e2);
     const Pair ab = f_bits(bx.h) >> 31 ? p_neg(bx) : bx;
     const Pair S2 = p_norm(p_sub(p_mul(ab, iq), sms));  // normalised: its sign is that of h
+    const float dv = fmaxf(fabsf(Dvy.h), fabsf(Dvz.h)), speed = fmaxf(fabsf(sms.h), ab.h * iq.h);
+    ok = ok && dv * fminf(w.h, 4.0f * speed) < kJump * w.h * w.h;
     const Pair a2 = p_neg_if(S2.h > 0.0f ? S2 : p_make(0.0f), !left);
     const Pair ahq = p_mul(a2, hq);
     ce = p_sub(ce, p_mul(ahq, e2));
